@@ -22,7 +22,7 @@ SOURCES = [
     "capi.cu",
     "kv_move.cu", "kv_gather_tma.cu",
     "mla_decode_simt.cu",
-    "mla_decode_tc.cu",
+    "mla_decode_tc.cu", "mla_decode_cluster.cu",
     "kv_block_pool.cpp",
     "kv_arena.cpp",
     "kv_partition.cpp",

@@ -63,6 +63,9 @@ bool TcPeerSupports(const b200kv_decode_args& a);
 int32_t LaunchMlaDecodeSimt(const b200kv_decode_args& a, cudaStream_t stream, int32_t* status);
 int32_t LaunchMlaDecodeTc(const b200kv_decode_args& a, int32_t n_ctas, cudaStream_t stream, int32_t* status,
                           const PeerRing* ring);
+int32_t TryDecodeCluster(const b200kv_decode_args& a, cudaStream_t stream, int32_t* status, bool* launched);
+bool ClusterSupportsAny(const b200kv_decode_args& a);
+int32_t LaunchDecodeClusterAny(const b200kv_decode_args& a, cudaStream_t stream, int32_t* status);
 int32_t LaunchLseMerge(const float* part_o, const float* part_m, const float* part_l, int32_t n_parts, int64_t rows,
                        void* out, float* lse, float* merged_o, float* merged_m, float* merged_l, cudaStream_t stream);
 
@@ -206,7 +209,16 @@ extern "C" int32_t b200kv_mla_decode(const b200kv_decode_args* args, void* strea
     SetLastError("decode: workspace of %zu bytes (16-byte aligned) required, %zu given", need, a.workspace_bytes);
     return a.workspace == nullptr ? B200KV_ERR_NULLPTR : B200KV_ERR_INVALID;
   }
-  if (use_tc) return LaunchMlaDecodeTc(a, ctas, static_cast<cudaStream_t>(stream), status, nullptr);
+  if (use_tc) {
+    bool launched = false;
+    if (int32_t rc = TryDecodeCluster(a, static_cast<cudaStream_t>(stream), status, &launched)) return rc;
+    return launched ? B200KV_OK : LaunchMlaDecodeTc(a, ctas, static_cast<cudaStream_t>(stream), status, nullptr);
+  }
+  // Any other geometry: the cluster kernel on tensor cores, unless the caller asks for the CUDA-core kernel, for fp32
+  // partials (whose weights that kernel keeps in fp32) or has a query the tensor cores cannot load.
+  if (a.variant == B200KV_DECODE_AUTO && ClusterSupportsAny(a)) {
+    return LaunchDecodeClusterAny(a, static_cast<cudaStream_t>(stream), status);
+  }
   b200kv_decode_args simt = a;
   if (a.row_index != nullptr) {  // the CUDA-core kernel reads a row list as a table of single-row blocks
     simt.block_table = a.row_index;

@@ -35,29 +35,16 @@
 
 #include "common.cuh"
 #include "kv_peer.cuh"
+#include "mla_tc_common.cuh"
 #include "sm100_ptx.cuh"
 
 namespace b200kv {
 
 namespace {
 
-constexpr int kHeads = 64;
-constexpr int kLatent = B200KV_LATENT_DIM;
-constexpr int kRope = B200KV_ROPE_DIM;
-constexpr int kTile = 64;      // tokens per tile / KV stage
-constexpr int kStages = 2;
-constexpr int kGroups = 4;                              // slab groups of a stage: slabs 2c, 2c+1 (and 8 with the last)
-constexpr int kSlabBytes = kTile * 128;                 // one 64-column slab of a tile: kTile rows x 128 B
-constexpr int kStageBytes = 9 * kSlabBytes;             // 73,728
-constexpr int kQSlabBytes = kHeads * 128;               // 8,192
-constexpr int kQBytes = 9 * kQSlabBytes;                // 73,728
-constexpr int kSoftmaxThreads = 128;
-constexpr int kSoftmaxWarps = kSoftmaxThreads / 32;     // one lane of each arrives on the barriers they signal
-constexpr int kThreads = 224;
-constexpr uint32_t kTmemCols = 512;
-constexpr uint32_t kTmemColS = 256;                     // S buffers at columns 256 and 256 + kTile
-constexpr float kRescaleThreshold = 8.0f;               // log2 units: rescale O only when max grows by > 2^8
+using namespace mla;
 
+constexpr int kThreads = 224;
 // Shared memory carve-up (offsets from a 1024-byte aligned base).
 constexpr int kOffQ = 0;
 constexpr int kOffKv = kOffQ + kQBytes;
@@ -139,54 +126,6 @@ struct TcParams {
   int32_t* status;
 };
 
-__device__ __forceinline__ int TilesOf(int len) { return (len + kTile - 1) / kTile; }
-
-__device__ __forceinline__ bool Aborting(const Misc* misc) {
-  return *reinterpret_cast<const volatile int32_t*>(&misc->abort_flag) != 0;
-}
-
-__device__ __noinline__ void RaiseTimeout(Misc* misc, int32_t* status, int site, uint32_t parity) {
-  *reinterpret_cast<volatile int32_t*>(&misc->abort_flag) = 1;
-  RecordError(status, B200KV_DEV_TIMEOUT, site, static_cast<int32_t>(blockIdx.x), static_cast<int32_t>(parity));
-}
-
-// Bounded mbarrier wait. Returns false when the CTA is aborting or this wait ran out (about one
-// second), after recording where.
-__device__ __noinline__ bool BoundedWait(uint32_t bar, uint32_t parity, Misc* misc, int32_t* status, int site) {
-  uint64_t start = 0;
-  for (uint32_t it = 0;; ++it) {
-    if (ptx::MbarTryWait(bar, parity)) return true;
-    if ((it & 255u) == 255u) {
-      if (Aborting(misc)) return false;
-      const uint64_t now = ptx::GlobalTimerNs();
-      if (start == 0) start = now;
-      if (now - start > 1000000000ull) {
-        RaiseTimeout(misc, status, site, parity);
-        return false;
-      }
-    }
-  }
-}
-
-// The same with a non-blocking probe in a tight loop. mbarrier.try_wait parks the thread and, measured here, a
-// parked thread resumes some 500 cycles after the phase completes; the producer's waits sit on the path that
-// refills a stage, so it spins instead (one thread: the issue slots it takes are few).
-__device__ __noinline__ bool BoundedSpin(uint32_t bar, uint32_t parity, Misc* misc, int32_t* status, int site) {
-  uint64_t start = 0;
-  for (uint32_t it = 0;; ++it) {
-    if (ptx::MbarTestWait(bar, parity)) return true;
-    if ((it & 1023u) == 1023u) {
-      if (Aborting(misc)) return false;
-      const uint64_t now = ptx::GlobalTimerNs();
-      if (start == 0) start = now;
-      if (now - start > 1000000000ull) {
-        RaiseTimeout(misc, status, site, parity);
-        return false;
-      }
-    }
-  }
-}
-
 // ---- work partition -----------------------------------------------------------------------------------
 // The tiles of all sequences form one flat list (sequence after sequence, empty ones contribute nothing).
 // Cutting that list into G equal runs of tiles leaves the CTAs uneven: a CTA whose run crosses from one
@@ -254,24 +193,6 @@ struct SegmentWalker {
     return false;
   }
 };
-
-// A 64-bit shared-memory descriptor whose start address is advanced by adding to the low word.
-__device__ __forceinline__ uint64_t DescAt(uint64_t base_desc, uint32_t byte_offset) {
-  return base_desc + static_cast<uint64_t>(byte_offset >> 4);
-}
-
-// The QK k-steps of kSlabs 64-column slabs (four each) starting at slab kFirstSlab; called by the whole MMA warp.
-template <int kFirstSlab, int kSlabs>
-__device__ __forceinline__ void IssueQkGroup(uint64_t q_desc, uint64_t kdesc, uint32_t d) {
-  constexpr uint32_t kIdescQk = ptx::InstrDescBf16(64, kTile, 0, 0);
-#pragma unroll
-  for (int i = 0; i < 4 * kSlabs; ++i) {
-    const int c = kFirstSlab + (i >> 2), kk = i & 3;
-    const uint64_t a = DescAt(q_desc, c * kQSlabBytes + kk * 32);
-    const uint64_t b = DescAt(kdesc, c * kSlabBytes + kk * 32);
-    if (ptx::ElectOne()) ptx::MmaF16SS(d, a, b, kIdescQk, (kFirstSlab + i) > 0 ? 1u : 0u);
-  }
-}
 
 // kGathered: the tiles are runs of 64 entries of a list of pool rows (TcParams::row_index) instead of runs of 64
 // tokens of a block; a separate instantiation, so that the dense kernel's code is not touched by it.
@@ -1533,6 +1454,8 @@ struct MapKeyHash {
   }
 };
 
+}  // namespace
+
 // Row-major [rows][width] bf16 view with row stride `stride` elements; box = 64 columns x box_rows rows (a tile
 // of 64 consecutive rows, or a single row for the loads that gather four rows each), 128-byte swizzle. Maps are
 // cached: a decode step reuses the same 2 x layers views every token.
@@ -1575,15 +1498,20 @@ int32_t GetRowMap(const void* base, int64_t stride, int64_t rows, int32_t width,
   return B200KV_OK;
 }
 
-// Query view [batch][64 heads][576] bf16 with element strides (q_seq_stride, q_head_stride, 1);
-// box = 64 columns x 64 heads of one sequence, 128-byte swizzle.
+// Query view [batch][heads][576] bf16 with element strides (q_seq_stride, q_head_stride, 1);
+// box = 64 columns x box_heads heads of one sequence (heads beyond the last read as zero), 128-byte swizzle.
+namespace {
+
 struct QKey {
   const void* base;
   int64_t head_stride;
   int64_t seq_stride;  // the effective one: a batch of one has none of its own
   int32_t batch;
+  int32_t heads;
+  int32_t box_heads;
   bool operator==(const QKey& o) const {
-    return base == o.base && head_stride == o.head_stride && seq_stride == o.seq_stride && batch == o.batch;
+    return base == o.base && head_stride == o.head_stride && seq_stride == o.seq_stride && batch == o.batch && heads == o.heads &&
+           box_heads == o.box_heads;
   }
 };
 struct QKeyHash {
@@ -1591,16 +1519,19 @@ struct QKeyHash {
     size_t h = reinterpret_cast<size_t>(k.base);
     h ^= static_cast<size_t>(k.head_stride) * 0x9E3779B97F4A7C15ull;
     h ^= static_cast<size_t>(k.seq_stride) * 0xC2B2AE3D27D4EB4Full;
-    return h ^ (static_cast<size_t>(k.batch) * 0x165667B19E3779F9ull);
+    return h ^ (static_cast<size_t>(k.batch) * 0x165667B19E3779F9ull) ^ (static_cast<size_t>(k.heads) << 32) ^ (static_cast<size_t>(k.box_heads) << 8);
   }
 };
 
-int32_t GetQMap(const void* base, int64_t head_stride, int64_t seq_stride, int32_t batch, CUtensorMap* out) {
+}  // namespace
+
+int32_t GetQMap(const void* base, int64_t head_stride, int64_t seq_stride, int32_t batch, int32_t heads, int32_t box_heads,
+                CUtensorMap* out) {
   static std::mutex mu;
   static std::unordered_map<QKey, CUtensorMap, QKeyHash> cache;
   // A batch of one has no meaningful sequence stride; any multiple of 16 bytes that covers a sequence will do.
-  const int64_t seq_stride_eff = batch > 1 ? seq_stride : static_cast<int64_t>(kHeads) * head_stride;
-  const QKey key{base, head_stride, seq_stride_eff, batch};
+  const int64_t seq_stride_eff = batch > 1 ? seq_stride : static_cast<int64_t>(heads) * head_stride;
+  const QKey key{base, head_stride, seq_stride_eff, batch, heads, box_heads};
   {
     std::lock_guard<std::mutex> lock(mu);
     auto it = cache.find(key);
@@ -1614,9 +1545,9 @@ int32_t GetQMap(const void* base, int64_t head_stride, int64_t seq_stride, int32
     SetLastError("cuTensorMapEncodeTiled could not be resolved from the CUDA driver");
     return B200KV_ERR_RUNTIME;
   }
-  const cuuint64_t dims[3] = {static_cast<cuuint64_t>(kLatent + kRope), kHeads, static_cast<cuuint64_t>(batch)};
+  const cuuint64_t dims[3] = {static_cast<cuuint64_t>(kLatent + kRope), static_cast<cuuint64_t>(heads), static_cast<cuuint64_t>(batch)};
   const cuuint64_t strides[2] = {static_cast<cuuint64_t>(head_stride) * 2, static_cast<cuuint64_t>(seq_stride_eff) * 2};
-  const cuuint32_t box[3] = {64, kHeads, 1};
+  const cuuint32_t box[3] = {64, static_cast<cuuint32_t>(box_heads), 1};
   const cuuint32_t elem[3] = {1, 1, 1};
   CUtensorMap map;
   const CUresult rc = encode(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box,
@@ -1636,8 +1567,6 @@ int32_t GetQMap(const void* base, int64_t head_stride, int64_t seq_stride, int32
   *out = map;
   return B200KV_OK;
 }
-
-}  // namespace
 
 // Row-major [rows][128] one-byte view (FP8 vectors of 128) with a row stride of `stride_bytes`; box = the whole
 // 128-byte row x box_rows rows, 128-byte swizzle. For the indexer's tensor-core kernel; encoded per call.
@@ -1700,10 +1629,8 @@ bool TcSupports(const b200kv_decode_args& a) {
 
 bool TcPeerSupports(const b200kv_decode_args& a) { return a.batch < 16; }
 
-// ring != nullptr: the call's sequences are KV-range shards and the merge kernel finishes them across the GPUs
-// (TcPeerSupports says for which batches that form exists).
-int32_t LaunchMlaDecodeTc(const b200kv_decode_args& a, int32_t n_ctas, cudaStream_t stream, int32_t* status,
-                          const PeerRing* ring) {
+// What the fused append needs, in either tensor-core kernel.
+int32_t CheckFusedAppend(const b200kv_decode_args& a) {
   if (a.new_latent != nullptr || a.new_rope != nullptr) {
     if (a.new_latent == nullptr || a.new_rope == nullptr) {
       SetLastError("decode: a fused append needs both new_latent and new_rope");
@@ -1718,6 +1645,14 @@ int32_t LaunchMlaDecodeTc(const b200kv_decode_args& a, int32_t n_ctas, cudaStrea
       return B200KV_ERR_INVALID;
     }
   }
+  return B200KV_OK;
+}
+
+// ring != nullptr: the call's sequences are KV-range shards and the merge kernel finishes them across the GPUs
+// (TcPeerSupports says for which batches that form exists).
+int32_t LaunchMlaDecodeTc(const b200kv_decode_args& a, int32_t n_ctas, cudaStream_t stream, int32_t* status,
+                          const PeerRing* ring) {
+  if (int32_t rc = CheckFusedAppend(a)) return rc;
   static thread_local int configured_device = -1;
   int device = 0;
   if (int32_t rc = CheckCuda(cudaGetDevice(&device), "cudaGetDevice")) return rc;
@@ -1740,7 +1675,7 @@ int32_t LaunchMlaDecodeTc(const b200kv_decode_args& a, int32_t n_ctas, cudaStrea
   if (int32_t rc = GetRowMap(a.pool.rope, a.pool.rope_row_stride, a.pool.pool_rows, kRope, box_rows, &rope_map)) return rc;
 
   CUtensorMap q_map;
-  if (int32_t rc = GetQMap(a.q, a.q_head_stride, a.q_seq_stride, a.batch, &q_map)) return rc;
+  if (int32_t rc = GetQMap(a.q, a.q_head_stride, a.q_seq_stride, a.batch, a.heads, kHeads, &q_map)) return rc;
 
   TcParams p{};
   p.q = static_cast<const __nv_bfloat16*>(a.q);

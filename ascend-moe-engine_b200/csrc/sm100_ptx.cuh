@@ -239,6 +239,16 @@ __device__ __forceinline__ void TmemLd32(uint32_t taddr, uint32_t (&r)[32]) {
       : "memory");
 }
 
+__device__ __forceinline__ void TmemLd16(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+}
+
 // 16 lanes x 64 columns spread over the whole warp (shape 16x256b, eight repetitions): thread t receives, for
 // each group i of eight columns, r[4i], r[4i+1] = lane t/4, columns 8i + 2(t%4) and the next, and r[4i+2],
 // r[4i+3] = lane t/4 + 8, same columns. An M=64 accumulator keeps its rows in lanes 0-15 of each 32-lane
@@ -300,6 +310,22 @@ __device__ __forceinline__ bool NamedBarrierOr(uint32_t id, uint32_t threads, bo
       : "r"(static_cast<uint32_t>(pred)), "r"(id), "r"(threads)
       : "memory");
   return out != 0;
+}
+
+// ---- thread-block clusters: barrier over all threads of all CTAs, and distributed shared memory ----
+__device__ __forceinline__ void ClusterArrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void ClusterWait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// The address, in the cluster's shared window, of `addr` of this CTA as the CTA of cluster rank `rank` has it.
+__device__ __forceinline__ uint32_t MapToRank(uint32_t addr, uint32_t rank) {
+  uint32_t out;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(out) : "r"(addr), "r"(rank));
+  return out;
+}
+__device__ __forceinline__ void StClusterF32(uint32_t addr, float v) {
+  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
+}
+__device__ __forceinline__ void StClusterV4(uint32_t addr, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
+  asm volatile("st.shared::cluster.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
 }
 
 __device__ __forceinline__ void StShared32(uint32_t addr, uint32_t v) {

@@ -1,0 +1,125 @@
+"""The cluster form of the decode attention (one launch, partials exchanged through distributed shared memory): every
+cluster size (the batch decides it), every split of a cluster into token and column ranges (the length decides it),
+tile edges, and the geometries that only this form serves on tensor cores (any block size, any head count)."""
+import numpy as np
+import pytest
+import torch
+
+import b200kv
+import kvo
+import scenarios
+from gpu_util import from_dev_bf16, run_decode, status_ok, to_dev_bf16, to_dev_i32
+
+pytestmark = pytest.mark.gpu
+
+NAN_BF16 = 0x7FC0
+EDGES = [1, 63, 64, 65, 128, 129, 192, 257, 320, 513, 640]
+
+
+def _pool_with_poison(kv_len, bs):
+    """A pool whose rows outside the sequences are NaN, and its tables."""
+    blocks = int(sum(scenarios.blocks_for(int(n), bs) for n in kv_len)) + 3
+    table = scenarios.build_tables(kv_len, bs, blocks, order=kvo.permutation(blocks))
+    pool = kvo.make_pool(blocks * bs)
+    owned = np.zeros(blocks * bs, dtype=bool)
+    for b, n in enumerate(kv_len):
+        j = np.arange(int(n))
+        owned[table[b, j // bs].astype(np.int64) * bs + j % bs] = True
+    owned[0] = True  # (a row past a sequence's end may be read as row 0, whose weight is then zero)
+    poisoned = pool.copy()
+    poisoned[~owned] = NAN_BF16
+    return pool, poisoned, table
+
+
+# batch -> cluster size: 1 .. 8 sequences 16 (or 8), then 8, 4, 2 and single CTAs
+@pytest.mark.parametrize("batch", [1, 2, 7, 12, 30, 60, 140])
+def test_small_batches_match_the_reference(batch):
+    bs = 64
+    kv_len = np.array([([512] + EDGES + [0])[(5 * i + batch) % 13] for i in range(batch)], dtype=np.int32)
+    if batch >= 140:
+        kv_len = np.minimum(kv_len, 512).astype(np.int32)  # table of eight tiles: still the cluster form with single CTAs
+    if not kv_len.any():
+        kv_len[0] = 65
+    pool, poisoned, table = _pool_with_poison(kv_len, bs)
+    q = kvo.make_q(batch, scale=2.0 / 24.0)
+    ref_out, ref_lse = scenarios.ref_attention_f64(q, pool, table, kv_len, bs, 1.0 / 24.0)
+    out, lse = run_decode(q, poisoned, table, kv_len, bs, 1.0 / 24.0, b200kv.DECODE_TCGEN05)
+    scenarios.check_attention(out, lse, ref_out, ref_lse, what=f"cluster batch {batch}")
+    assert (out[kv_len == 0] == 0).all()
+
+
+@pytest.mark.parametrize("length", [1, 64, 100, 129, 257, 512, 513, 1024, 2048, 8192])
+def test_one_sequence_of_every_split(length):
+    """Up to 8,192 tokens one sequence takes a cluster of 16: 4 x 4, 8 x 2 and 16 x 1 token x column ranges."""
+    kv_len = np.array([length], dtype=np.int32)
+    pool, poisoned, table = _pool_with_poison(kv_len, 128)
+    q = kvo.make_q(1)
+    ref_out, ref_lse = scenarios.ref_attention_f64(q, pool, table, kv_len, 128, 1.0 / 24.0)
+    out, lse = run_decode(q, poisoned, table, kv_len, 128, 1.0 / 24.0, b200kv.DECODE_TCGEN05)
+    scenarios.check_attention(out, lse, ref_out, ref_lse, what=f"cluster length {length}", strict_abs=True)
+    po, pm, pl = run_decode(q, poisoned, table, kv_len, 128, 1.0 / 24.0, b200kv.DECODE_TCGEN05, partial=True)
+    scenarios.check_attention(kvo.f32_to_bf16(po / pl[..., None]), pm + np.log(pl), ref_out, ref_lse,
+                              what=f"cluster partial {length}", strict_abs=True)
+
+
+@pytest.mark.parametrize("kv_len", [[1], [129], [64, 65, 1, 700], [128] * 40])
+def test_fused_append_and_quantisation(kv_len):
+    """The CTAs of every column range write the new row before they load its tile; the quantised bytes are those of the
+    stand-alone quantiser on the output."""
+    bs, batch = 64, len(kv_len)
+    kv_len = np.array(kv_len, dtype=np.int32)
+    pool, _, table = _pool_with_poison(kv_len, bs)
+    latent, rope = kvo.normal_bf16(batch * 512, 21).reshape(batch, 512), kvo.normal_bf16(batch * 64, 22).reshape(batch, 64)
+    want = pool.copy()
+    last = kv_len.astype(np.int64) - 1
+    rows = table[np.arange(batch), last // bs].astype(np.int64) * bs + last % bs
+    want[rows, :512], want[rows, 512:] = latent, rope
+    q = kvo.make_q(batch)
+    ref_out, ref_lse = scenarios.ref_attention_f64(q, want, table, kv_len, bs, 1.0 / 24.0)
+    d_pool, status = to_dev_bf16(pool), b200kv.new_status()
+    out = torch.empty((batch, 64, 512), dtype=torch.bfloat16, device="cuda")
+    lse = torch.empty((batch, 64), dtype=torch.float32, device="cuda")
+    fp8 = torch.empty((batch, 64, 512), dtype=torch.uint8, device="cuda")
+    scales = torch.empty((batch, 64, 16), dtype=torch.uint8, device="cuda")
+    ws = torch.empty(b200kv.decode_workspace_bytes(batch), dtype=torch.uint8, device="cuda")
+    b200kv.mla_decode(to_dev_bf16(q), b200kv.pool_view(d_pool), to_dev_i32(table), to_dev_i32(kv_len), bs, 1.0 / 24.0, out=out, lse=lse,
+                      workspace=ws, status=status, new_rows=(to_dev_bf16(latent), to_dev_bf16(rope)), stable_tables=True,
+                      quantised=(fp8, scales))
+    status_ok(status)
+    assert np.array_equal(from_dev_bf16(d_pool), want)
+    # sequences of one token have outputs of magnitude 3: the per-row bound, not the absolute one
+    scenarios.check_attention(from_dev_bf16(out), lse.cpu().numpy(), ref_out, ref_lse, what="cluster append")
+    fp8_2, scales_2 = torch.empty((batch, 64 * 512), dtype=torch.uint8, device="cuda"), torch.empty((batch, 1024), dtype=torch.uint8, device="cuda")
+    b200kv.mx_quant_e4m3(out.view(batch, -1), fp8_2, scales_2)
+    assert torch.equal(fp8.view(batch, -1), fp8_2) and torch.equal(scales.view(batch, -1), scales_2)
+
+
+@pytest.mark.parametrize("heads,bs", [(64, 16), (64, 1), (64, 48), (64, 96), (1, 64), (5, 16), (16, 64), (63, 32), (65, 64), (128, 16)])
+def test_any_geometry_is_as_exact_as_the_cuda_core_kernel(heads, bs):
+    """Block sizes that are no multiple of 64 and head counts other than 64: against the float64 reference, and no
+    further from it than the CUDA-core kernel with its fp32 weights. Both results are bf16, whose rounding is 2^-9 of a
+    value at most; the split weights add 2^-17, so the mean errors agree far within 10 %."""
+    kv_len = np.array([1, 17, 64, 65, 1000, 0, 333], dtype=np.int32)
+    pool, poisoned, table = _pool_with_poison(kv_len, bs)
+    q = kvo.make_q(len(kv_len), heads=heads, scale=0.3)
+    ref_out, ref_lse = scenarios.ref_attention_f64(q, pool, table, kv_len, bs, 1.0 / 24.0)
+    out, lse = run_decode(q, poisoned, table, kv_len, bs, 1.0 / 24.0, b200kv.DECODE_AUTO)
+    scenarios.check_attention(out, lse, ref_out, ref_lse, what=f"any geometry {heads} x {bs}")
+    simt, _ = run_decode(q, poisoned, table, kv_len, bs, 1.0 / 24.0, b200kv.DECODE_SIMT)
+    live = kv_len > 0
+    err = np.abs(kvo.bf16_to_f32(out[live]).astype(np.float64) - ref_out[live]).mean()
+    err_simt = np.abs(kvo.bf16_to_f32(simt[live]).astype(np.float64) - ref_out[live]).mean()
+    assert err <= 1.1 * err_simt, (err, err_simt)
+
+
+def test_any_geometry_reports_a_length_beyond_the_table():
+    bs = 16
+    pool, _, table = _pool_with_poison(np.array([200, 64], dtype=np.int32), bs)
+    status = b200kv.new_status()
+    out = torch.empty((2, 64, 512), dtype=torch.bfloat16, device="cuda")
+    ws = torch.empty(b200kv.decode_workspace_bytes(2), dtype=torch.uint8, device="cuda")
+    b200kv.mla_decode(to_dev_bf16(kvo.make_q(2)), b200kv.pool_view(to_dev_bf16(pool)), to_dev_i32(table),
+                      to_dev_i32([200, bs * table.shape[1] + 40]), bs, 1.0 / 24.0, out=out, workspace=ws, status=status)
+    torch.cuda.synchronize()
+    got = status.cpu().tolist()
+    assert got[0] == b200kv.DEV_BAD_BLOCK and got[1] == 1, got
