@@ -23,7 +23,10 @@
 //
 // kSplitP: the softmax weights go to the tensor cores as two bf16 terms (P = hi + lo, 16 bits of it) instead of one,
 // for the geometries whose other kernel keeps them in fp32 (any page size, any head count): twice the PV instructions
-// for an error of 2^-17 of a weight, which the bf16 result does not show.
+// for an error of 2^-17 of a weight, which the bf16 result does not show. The tensor core truncates its fp32 running sum
+// after every K = 16 step, 36 of them for a score, a bias that the log-sum-exp keeps (5e-7 of it, where fp32 fmas are off
+// by 1.7e-7); so here each slab group of Q.K has an accumulator of its own (8 to 12 steps) and the four are added in
+// fp32, at the price of S being single-buffered.
 //
 // Measured (B200, graph of layers, us a layer): one sequence of 129 tokens with the append 16.4 (flat kernel and merge)
 // -> 7.9, of which 0.9 from the previous layer's end to the wait's return, 0.4 issue, 1.1 latency, 1.1 QK behind the
@@ -497,10 +500,11 @@ __global__ void __launch_bounds__(kThreads, 1)
     const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem, 0);
     const int n_u = __shfl_sync(0xffffffffu, n, 0);
     for (int i = 0; i < n_u && ok; ++i) {
-      const int stage = i % kStages, buf = i & 1;
+      const int stage = i % kStages, buf = kSplitP ? 0 : i & 1;
       const uint32_t kv_parity = (i / kStages) & 1;
       const uint64_t kdesc = DescAt(k_desc0, stage * kStageBytes);
       const uint32_t d = tmem_u + kTmemColS + kTile * buf;
+      constexpr uint32_t kNext = kSplitP ? kTile : 0;  // kSplitP: an accumulator per slab group
       auto group_ready = [&](int c) {
         ok = WarpSpin(bar(&misc->kv_full[stage][c]), kv_parity, misc, p.status, 224 + c);
         if (ok && i == 0) ok = WarpSpin(bar(&misc->q_full[c]), 0, misc, p.status, 222);
@@ -509,19 +513,19 @@ __global__ void __launch_bounds__(kThreads, 1)
         ptx::TcFenceAfterSync();
         if constexpr (kCopied) ptx::FenceProxyAsyncShared();
       };
-      if (i >= 2) ok = WarpSpin(bar(&misc->s_empty[buf]), ((i >> 1) & 1) ^ 1, misc, p.status, 228);
+      if (i >= (kSplitP ? 1 : 2)) ok = WarpSpin(bar(&misc->s_empty[buf]), ((kSplitP ? i : i >> 1) & 1) ^ 1, misc, p.status, 228);
       if (ok) group_ready(0);
       if (!ok) break;
-      IssueQkGroup<0, 2>(q_desc, kdesc, d);
+      IssueQkGroup<0, 2, kSplitP>(q_desc, kdesc, d);
       group_ready(1);
       if (!ok) break;
-      IssueQkGroup<2, 2>(q_desc, kdesc, d);
+      IssueQkGroup<2, 2, kSplitP>(q_desc, kdesc, d + kNext);
       group_ready(2);
       if (!ok) break;
-      IssueQkGroup<4, 2>(q_desc, kdesc, d);
+      IssueQkGroup<4, 2, kSplitP>(q_desc, kdesc, d + 2 * kNext);
       group_ready(3);
       if (!ok) break;
-      IssueQkGroup<6, 3>(q_desc, kdesc, d);
+      IssueQkGroup<6, 3, kSplitP>(q_desc, kdesc, d + 3 * kNext);
       if (ptx::ElectOne()) ptx::TcCommit(bar(&misc->s_full[buf]));
     }
   } else if (warp == 6 && n > 0) {
@@ -577,15 +581,25 @@ __global__ void __launch_bounds__(kThreads, 1)
     const uint32_t lane_base = static_cast<uint32_t>(warp * 32) << 16;
     const bool has_rows = warp * 16 < share.heads;  // otherwise the warp only keeps step with the others
     for (int i = 0; i < n; ++i) {
-      const int buf = i & 1, stage = i % kStages;
+      const int buf = kSplitP ? 0 : i & 1, stage = i % kStages;
       const int valid = min(kTile, len - (share.t_lo + i) * kTile);
-      ok = WarpSpin(bar(&misc->s_full[buf]), (i >> 1) & 1, misc, p.status, 230);
+      ok = WarpSpin(bar(&misc->s_full[buf]), (kSplitP ? i : i >> 1) & 1, misc, p.status, 230);
       if (!ok) break;
       ptx::TcFenceAfterSync();
       uint32_t sr[32];
       if (has_rows) {
         ptx::TmemLd16x256bX8(tmem + lane_base + kTmemColS + kTile * buf, sr);
         ptx::TmemWaitLd();
+        if constexpr (kSplitP) {
+#pragma unroll 1
+          for (int c = 1; c < kGroups; ++c) {
+            uint32_t more[32];
+            ptx::TmemLd16x256bX8(tmem + lane_base + kTmemColS + kTile * c, more);
+            ptx::TmemWaitLd();
+#pragma unroll
+            for (int j = 0; j < 32; ++j) sr[j] = __float_as_uint(__uint_as_float(sr[j]) + __uint_as_float(more[j]));
+          }
+        }
       } else {
 #pragma unroll
         for (int j = 0; j < 32; ++j) sr[j] = 0u;

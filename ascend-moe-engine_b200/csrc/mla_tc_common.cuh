@@ -85,7 +85,8 @@ __device__ __forceinline__ uint64_t DescAt(uint64_t base_desc, uint32_t byte_off
 }
 
 // The QK k-steps of kSlabs 64-column slabs (four each) starting at slab kFirstSlab; called by the whole MMA warp.
-template <int kFirstSlab, int kSlabs>
+// kFresh: the group starts an accumulator of its own instead of adding to what the groups before it left.
+template <int kFirstSlab, int kSlabs, bool kFresh = false>
 __device__ __forceinline__ void IssueQkGroup(uint64_t q_desc, uint64_t kdesc, uint32_t d) {
   constexpr uint32_t kIdescQk = ptx::InstrDescBf16(64, kTile, 0, 0);
 #pragma unroll
@@ -93,7 +94,7 @@ __device__ __forceinline__ void IssueQkGroup(uint64_t q_desc, uint64_t kdesc, ui
     const int c = kFirstSlab + (i >> 2), kk = i & 3;
     const uint64_t a = DescAt(q_desc, c * kQSlabBytes + kk * 32);
     const uint64_t b = DescAt(kdesc, c * kSlabBytes + kk * 32);
-    if (ptx::ElectOne()) ptx::MmaF16SS(d, a, b, kIdescQk, (kFirstSlab + i) > 0 ? 1u : 0u);
+    if (ptx::ElectOne()) ptx::MmaF16SS(d, a, b, kIdescQk, (kFresh ? i : kFirstSlab + i) > 0 ? 1u : 0u);
   }
 }
 
