@@ -45,7 +45,8 @@ constexpr int kThreads = 320;
 constexpr int kEpilogueThreads = 128;  // per group
 constexpr int kProducerWarp = 8, kMmaWarp = 9;
 constexpr int kTmemCols = 128;     // two accumulators of 64 columns
-constexpr int kSmemBytes = kStages * kStageBytes + 1024 /* alignment */ + 2048 /* barriers, scalars, coefficients */;
+constexpr int kTailBytes = 3072;   // barriers, scalars, coefficients
+constexpr int kSmemBytes = kStages * kStageBytes + 1024 /* alignment */ + kTailBytes;
 
 struct TcScoreParams {
   const float* q_scale;    // [B][heads]
@@ -63,7 +64,7 @@ struct TcScoreParams {
   int32_t* status;
 };
 
-struct Shared {  // at most 2048 bytes
+struct Shared {  // at most kTailBytes
   uint64_t full[kStages];
   uint64_t empty[kStages];
   uint64_t acc_full[2];
@@ -71,11 +72,14 @@ struct Shared {  // at most 2048 bytes
   uint32_t tmem_base;
   int32_t abort_flag;
   int32_t start_seq, start_tile, n_tiles;
-  alignas(16) float qs[2][kHeadsPadded];
-  alignas(16) float w[2][kHeadsPadded];
+  // Per epilogue group, and per parity of the group's tiles: a warp that is done with a tile writes the next tile's
+  // coefficients while a slower one still reads this tile's. (It cannot get two tiles ahead: between them lies the
+  // group's barrier.)
+  alignas(16) float qs[2][2][kHeadsPadded];
+  alignas(16) float w[2][2][kHeadsPadded];
 };
 
-static_assert(sizeof(Shared) <= 2048, "the tail of the shared-memory budget");
+static_assert(sizeof(Shared) <= kTailBytes, "the tail of the shared-memory budget");
 
 __device__ __forceinline__ int TilesOf(int len) { return len > 0 ? (len + kTokens - 1) / kTokens : 0; }
 
@@ -341,8 +345,8 @@ __global__ void __launch_bounds__(kThreads, 1)
       cur = next;
       have = fetch(&next);
       if (gtid < kHeadsPadded) {
-        sh->qs[buf][gtid] = cur.qs;
-        sh->w[buf][gtid] = cur.w;
+        sh->qs[buf][n & 1][gtid] = cur.qs;
+        sh->w[buf][n & 1][gtid] = cur.w;
       }
       ptx::NamedBarrier(1 + group, kEpilogueThreads);
       ok = __all_sync(0xffffffffu, Wait(bar(&sh->acc_full[buf]), n & 1, sh, p.status, 3));
@@ -357,8 +361,8 @@ __global__ void __launch_bounds__(kThreads, 1)
       __syncwarp();
       if (lane == 0) ptx::MbarArrive(bar(&sh->acc_empty[buf]));
       float score = 0.0f;
-      const float4* qs4 = reinterpret_cast<const float4*>(sh->qs[buf]);
-      const float4* w4 = reinterpret_cast<const float4*>(sh->w[buf]);
+      const float4* qs4 = reinterpret_cast<const float4*>(sh->qs[buf][n & 1]);
+      const float4* w4 = reinterpret_cast<const float4*>(sh->w[buf][n & 1]);
       // A head beyond the sequence's count is skipped, not multiplied by a zero weight: its column of the
       // accumulator came from rows of Q that belong to the next sequence (or from nothing) and may hold anything.
       auto head = [&](int h, float qs_h, float w_h, uint32_t dot) {

@@ -311,6 +311,30 @@ def test_indexer_tensor_core_scores_and_selection(lens, heads, k):
                                     kv_len, k, eps_rel=1e-6)
 
 
+def test_indexer_tensor_core_scores_where_a_run_crosses_into_the_next_sequence():
+    """32 sequences of about 4,000 tokens on 148 CTAs: most CTAs' runs of tiles cross from one sequence into the next,
+    whose per-head coefficients differ. Every score, in each of 30 calls, against the CUDA-core kernel's."""
+    B, heads, bs, k = 32, 64, 64, 16
+    g = torch.Generator(device="cuda")
+    g.manual_seed(20251008)
+    lens = torch.randint(3300, 4097, (B,), generator=g, device="cuda", dtype=torch.int32)
+    blocks = 4096 // bs
+    table = torch.randperm(B * blocks, generator=g, device="cuda").to(torch.int32).view(B, blocks)
+    fp8 = lambda *shape: torch.randn(shape, generator=g, device="cuda").to(torch.float8_e4m3fn).view(torch.uint8)
+    q, key = fp8(B, heads, 128), fp8(B * blocks * bs, 128)
+    qs = torch.rand((B, heads), generator=g, device="cuda") * 0.03 + 0.001
+    w = torch.randn((B, heads), generator=g, device="cuda").bfloat16()
+    ks = torch.rand((B * blocks * bs,), generator=g, device="cuda") * 0.02 + 0.01
+    want = []
+    b200kv.indexer_topk(q, qs, w, key, ks, table, lens, bs, 4096, k, variant=b200kv.INDEXER_EXACT, scores_out=want)
+    live = torch.arange(4096, device="cuda")[None, :] < lens[:, None]
+    bound = 1e-6 * torch.where(live, want[0], 0).abs().amax(dim=1, keepdim=True)
+    for _ in range(30):
+        got = []
+        b200kv.indexer_topk(q, qs, w, key, ks, table, lens, bs, 4096, k, variant=b200kv.INDEXER_TCGEN05, scores_out=got)
+        assert not (((got[0] - want[0]).abs() > bound) & live).any()
+
+
 def test_indexer_tensor_core_variant_is_refused_where_it_cannot_run_and_reports_bad_blocks():
     B, heads, bs, k = 2, 64, 64, 16
     q, qs, w, key, ks, table, kv_len = _indexer_inputs(B, heads, [200, 64], bs, seed=5)
