@@ -9,11 +9,12 @@
 // is kv_indexer_tc.cu; b200kv_indexer_topk chooses). The arithmetic is fixed
 // to the operation (one thread owns a token and runs the same fp32 fma chains as the CPU statement: over
 // d = 0..127 for each head, then over the heads), so scores are bit-identical with the oracle and the
-// selection is exact: tokens are ordered by (score descending, position ascending) as 64-bit keys; a radix
-// select finds the k-th key and a bitonic sort in shared memory orders the k that are taken.
+// selection is exact: tokens are ordered by (score descending, position ascending) as 64-bit keys; histograms find the
+// k-th key's neighbourhood, and the keys up to there are sorted.
 #include <cuda_fp8.h>
 
 #include "common.cuh"
+#include "sm100_ptx.cuh"
 
 namespace b200kv {
 namespace {
@@ -123,250 +124,447 @@ __device__ __forceinline__ uint64_t SortKey(float score, uint32_t position) {
   return (static_cast<uint64_t>(~bits) << 32) | position;
 }
 
-// One CTA per sequence. The k best tokens are the k smallest 64-bit keys, all distinct. A radix select finds
-// the k-th smallest key: the key's bits from the top in digits of 11, 11, 10 (the score) and 11, 11, 10 (the
-// position), each pass a histogram of the digit over the tokens that match the digits found so far, a block scan
-// of the histogram, and the digit in which the wanted rank falls. The passes stop as soon as every token that
-// still matches is wanted (with distinct scores: after the three score digits). Tokens whose key is at most
-// the one found are then collected, exactly k of them, and sorted (bitonic, the short-range steps on registers).
-// A thread keeps the score images of its first eight tokens
-// in registers, so sequences of up to 8,192 tokens are read from memory once; work is linear in the length.
-constexpr int kRadixBins = 2048;
-constexpr int kBinsPerThread = kRadixBins / kSortThreads;
+// The selection. The k best tokens are the k smallest 64-bit keys, all distinct. A cluster of C CTAs (1 .. 16, one for
+// every 4,096 tokens of the longest sequence, as long as the batch fits the GPU at once) takes a sequence, a CTA a
+// consecutive C-th of it, the score images of its first 8,192 tokens in registers.
+//
+//   bound    The k-th key is narrowed down by histograms of 512 bins over the range in which it lies, the first range
+//            being that of the sequence's scores (equal steps of the image between the smallest and the largest, so the
+//            bins that matter are thinly filled; bins of leading bits would put nearly all scores of a sequence into a
+//            handful). Every CTA reads the others' histograms through distributed shared memory and draws the same
+//            conclusion. The passes end when the keys up to the chosen bin's end are few enough to be sorted (half as
+//            many again as wanted): one pass for scores without far outliers. Scores that are equal
+//            are told apart by position, in histograms of positions, only when there are too many of them.
+//   collect  The histograms also say where each bin's keys belong in the order and which part of a bin is which CTA's, so
+//            a CTA can write its keys up to the bound straight to their bins' places in the list.
+//   order    Inside a bin the list is in no order: a key's place is its bin's start plus the number of smaller keys in the
+//            bin. The CTAs share the list's entries out (a key is sent to those whose entries its bin overlaps: small
+//            stores to another SM go at one in three or four cycles, so sending all to all took 4 us), several threads to
+//            a key. Bins hold tens of keys, so this is a few thousand comparisons a CTA in place of a sort; where scores
+//            are so equal that bins get large, one CTA sorts the list.
+//
+// Bound by latencies: a cluster barrier costs some 0.6 us and there are three. It replaces a radix select by leading
+// digits in one CTA (sequences up to 8,192 tokens; atomics on a few bins serialise), and for longer sequences in two
+// levels, of which the second, one CTA among the candidates of all chunks, took the most time.
+constexpr int kBins = 512;
+constexpr int kBinsLog2 = 9;
 constexpr int kHeldPerThread = 8;
-constexpr int kSelectChunk = kHeldPerThread * kSortThreads;  // 8,192 tokens: what one CTA reads once and keeps
+constexpr int kListKeys = 4096;  // keys that can be collected
+constexpr int kMaxCluster = 16;
+constexpr int kTokensPerCta = 4096;
+constexpr uint32_t kMostComparisons = 400000;  // per CTA, some 6 us of it: what sorting the list takes
 
-// Long sequences in two levels, so that more than one CTA works on a sequence: the k best of every chunk of
-// 8,192 tokens (kLevel 1: one CTA a chunk, its keys written unsorted to the candidate area), then the k best
-// of the candidates (kLevel 2: one CTA a sequence, elements are the 64-bit keys themselves). The k best of the
-// whole are among the k best of each chunk, so the result is that of one level (kLevel 0), which sequences of
-// up to a chunk use.
 struct SelectParams {
   const float* scores;
   int64_t score_stride;
   const int32_t* kv_len;
   int32_t k;
-  int32_t chunks;           // per sequence (levels 1 and 2)
-  uint64_t* candidates;     // [batch][chunks][k] keys (levels 1 and 2)
-  int32_t* index;           // [batch][k]
-  int32_t* n_selected;      // [batch]
+  int32_t* index;       // [batch][k]
+  int32_t* n_selected;  // [batch]
   const int32_t* block_table;
   int64_t max_blocks;
   int32_t block_size;
   int64_t pool_rows;
-  int32_t* rows_out;        // [batch][k] or null
+  int32_t* rows_out;    // [batch][k] or null
   int32_t* status;
 };
 
-template <int kLevel>
-__global__ void __launch_bounds__(kSortThreads) IndexerSelectKernel(SelectParams p) {
-  GridDependencyTrigger();
-  __shared__ uint64_t keys[kMaxK];
-  __shared__ uint32_t hist[kRadixBins];
-  __shared__ uint32_t warp_sum[32];
-  __shared__ uint32_t chosen[2][3];  // per pass parity: digit, elements before it, elements in it
-  __shared__ uint32_t n_taken;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  for (int i = tid; i < kRadixBins; i += kSortThreads) hist[i] = 0;
-  if (tid == 0) n_taken = 0;
-  GridDependencyWait();
-  const int b = kLevel == 1 ? blockIdx.y : blockIdx.x;
-  const int chunk = kLevel == 1 ? blockIdx.x : 0;
-  const int len = p.kv_len[b];
-  const int k = p.k;
-  // The elements this CTA selects among, n of them, and how many it keeps.
-  const int first = kLevel == 1 ? chunk * kSelectChunk : 0;  // first token (levels 0 and 1)
-  int n;
-  if (kLevel == 0) {
-    n = len;
-  } else if (kLevel == 1) {
-    n = len - first < kSelectChunk ? len - first : kSelectChunk;
-    if (n < 0) n = 0;
-  } else {
-    n = p.chunks * k;
+struct SelectShared {
+  uint64_t all[kListKeys];      // the list: the keys up to the bound, bin after bin; filled where this CTA's entries' bins lie
+  uint64_t scratch[kListKeys];  // this CTA's keys on their way to the lists; the sort's other buffer
+  uint16_t place[kListKeys];    // ... and where they go
+  alignas(16) uint32_t hist[2][kBins];  // by parity of the pass: the peers read one while the next is cleared
+  alignas(16) uint32_t peers[kMaxCluster][kBins];
+  uint32_t start[kBins + 1];  // place of a bin's first key in the list
+  uint32_t next[kBins + 1];   // place of this CTA's next key of a bin; entry kBins: of the keys below the last range
+  uint32_t n_mine;
+  uint32_t lo[kMaxCluster], hi[kMaxCluster];  // smallest and largest image of each CTA
+  uint32_t below[kMaxCluster];                // each CTA's keys below the last range
+  uint32_t warp_a[32], warp_b[32];
+  uint32_t chosen[3];  // bin, keys in the bins before it, keys in it
+};
+
+// Bitonic sort, ascending, of kEach * threads keys (a power of two; threads <= 1024, a multiple of 32, the block's first
+// ones): keys tid + j * threads of `data` in register j. Partners `threads` or more away sit in the same thread, less than
+// 32 away in the same warp; the others are exchanged through the two buffers in turn, one barrier a step.
+template <int kEach>
+__device__ void SortKeys(uint64_t* data, uint64_t* other, int threads) {
+  const int tid = threadIdx.x;
+  const int total = kEach * threads;
+  uint64_t key[kEach];
+#pragma unroll
+  for (int j = 0; j < kEach; ++j) key[j] = data[tid + j * threads];
+  asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory");
+  uint64_t* buffer = data;
+  for (int size = 2; size <= total; size <<= 1) {
+    for (int stride = size >> 1; stride > 0; stride >>= 1) {
+      if (stride >= threads) {
+        if constexpr (kEach > 1) {
+          const int apart = stride / threads;  // 1 or 2
+#pragma unroll
+          for (int j = 0; j < kEach; ++j) {
+#pragma unroll
+            for (int a = 1; a < kEach; a <<= 1) {
+              if (a == apart && (j & a) == 0) {
+                const bool ascending = ((tid + j * threads) & size) == 0;
+                const uint64_t x = key[j], y = key[j | a];
+                const bool swap = (x > y) == ascending;
+                key[j] = swap ? y : x;
+                key[j | a] = swap ? x : y;
+              }
+            }
+          }
+        }
+        continue;
+      }
+      if (stride >= 32) {
+#pragma unroll
+        for (int j = 0; j < kEach; ++j) buffer[tid + j * threads] = key[j];
+        asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory");
+      }
+#pragma unroll
+      for (int j = 0; j < kEach; ++j) {
+        const int e = tid + j * threads;
+        const uint64_t theirs = stride >= 32 ? buffer[e ^ stride] : __shfl_xor_sync(0xffffffffu, key[j], stride);
+        const bool keep_smaller = ((e & stride) == 0) == ((e & size) == 0);
+        if (keep_smaller ? theirs < key[j] : theirs > key[j]) key[j] = theirs;
+      }
+      if (stride >= 32) buffer = buffer == data ? other : data;
+    }
   }
-  const int kept = kLevel == 2 ? (len < k ? len : k) : (n < k ? n : k);
-  const float* row = p.scores + b * p.score_stride + first;
-  const uint64_t* cand_in = p.candidates + static_cast<int64_t>(b) * p.chunks * k;
-  uint64_t* cand_out = p.candidates + (static_cast<int64_t>(b) * p.chunks + chunk) * k;
-  if (kLevel != 1) {
+  asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory");
+#pragma unroll
+  for (int j = 0; j < kEach; ++j) data[tid + j * threads] = key[j];
+}
+
+__global__ void __launch_bounds__(kSortThreads) IndexerSelectKernel(SelectParams p) {
+  extern __shared__ __align__(16) unsigned char select_smem[];
+  SelectShared& sh = *reinterpret_cast<SelectShared*>(select_smem);
+  GridDependencyTrigger();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int cluster = gridDim.x, rank = blockIdx.x, b = blockIdx.y;
+  const int cluster_log2 = 31 - __clz(cluster);
+  auto cluster_sync = [&]() {
+    if (cluster > 1) {
+      __syncwarp();
+      ptx::ClusterArrive();
+      ptx::ClusterWait();
+    } else {
+      __syncthreads();
+    }
+  };
+  static_assert(2 * kBins <= kSortThreads, "one thread clears one bin");
+  if (tid < 2 * kBins) sh.hist[tid / kBins][tid % kBins] = 0;
+  if (tid == 0) sh.n_mine = 0;
+  if (cluster > 1) {
+    __syncwarp();
+    ptx::ClusterArrive();  // (waited for before the first exchange: the peers have started)
+  }
+  GridDependencyWait();
+  const int len = max(p.kv_len[b], 0);
+  const int k = p.k;
+  const int kept = min(len, k);
+  if (rank == 0) {
     if (tid == 0) p.n_selected[b] = kept;
     for (int i = kept + tid; i < k; i += kSortThreads) {
       p.index[b * k + i] = -1;
       if (p.rows_out != nullptr) p.rows_out[b * k + i] = -1;
     }
-  } else {
-    for (int i = kept + tid; i < k; i += kSortThreads) cand_out[i] = ~0ull;  // empties sort last
   }
-  if (kept == 0) return;
-  // Levels 0 and 1: the high word of the key (ascending = better) of this thread's elements tid, tid + 1024, ...,
-  // the first eight held in registers. Level 2 reads its few keys from memory every time.
+  if (kept == 0) {  // all CTAs of the cluster
+    if (cluster > 1) ptx::ClusterWait();
+    return;
+  }
+  const int per = (len + cluster - 1) >> cluster_log2;
+  const int first = min(rank * per, len);
+  const int n = min(per, len - first);
+  const float* row = p.scores + b * p.score_stride + first;
+  // The high word of the key (ascending = better) of this thread's elements tid, tid + 1024, ..., the first eight held.
   uint32_t held[kHeldPerThread];
-  if (kLevel != 2) {
+#pragma unroll
+  for (int j = 0; j < kHeldPerThread; ++j) {
+    const int e = tid + j * kSortThreads;
+    held[j] = e < n ? static_cast<uint32_t>(SortKey(row[e], 0u) >> 32) : 0u;
+  }
+  auto for_each = [&](auto&& body) {  // image and position of every element of this thread
 #pragma unroll
     for (int j = 0; j < kHeldPerThread; ++j) {
+      if (j * kSortThreads >= n) break;
       const int e = tid + j * kSortThreads;
-      held[j] = e < n ? static_cast<uint32_t>(SortKey(row[e], 0u) >> 32) : 0u;
+      if (e < n) body(held[j], static_cast<uint32_t>(first + e));
+    }
+    for (int e = tid + kHeldPerThread * kSortThreads; e < n; e += kSortThreads) {
+      body(static_cast<uint32_t>(SortKey(row[e], 0u) >> 32), static_cast<uint32_t>(first + e));
+    }
+  };
+
+  uint32_t img_lo = ~0u, img_hi = 0u;
+  for_each([&](uint32_t image, uint32_t) {
+    img_lo = min(img_lo, image);
+    img_hi = max(img_hi, image);
+  });
+  img_lo = __reduce_min_sync(0xffffffffu, img_lo);
+  img_hi = __reduce_max_sync(0xffffffffu, img_hi);
+  if (lane == 0) {
+    sh.warp_a[warp] = img_lo;
+    sh.warp_b[warp] = img_hi;
+  }
+  __syncthreads();
+  if (cluster > 1) ptx::ClusterWait();
+  if (warp == 0) {
+    img_lo = __reduce_min_sync(0xffffffffu, sh.warp_a[lane]);
+    img_hi = __reduce_max_sync(0xffffffffu, sh.warp_b[lane]);
+    if (lane < cluster) {
+      ptx::StClusterB32(ptx::MapToRank(ptx::SmemAddr(&sh.lo[rank]), lane), img_lo);
+      ptx::StClusterB32(ptx::MapToRank(ptx::SmemAddr(&sh.hi[rank]), lane), img_hi);
     }
   }
-  auto held_key = [&](int j, int e) -> uint64_t {  // j = e / 1024 (compile-time inside unrolled loops)
-    return (static_cast<uint64_t>(held[j]) << 32) | static_cast<uint32_t>(first + e);
-  };
-  auto read_key = [&](int e) -> uint64_t {
-    return kLevel == 2 ? cand_in[e] : SortKey(row[e], static_cast<uint32_t>(first + e));
-  };
-  constexpr int kFirstRead = kLevel == 2 ? 0 : kSelectChunk;  // elements from here on are read, not held
-  __syncthreads();  // the histogram is clear
+  cluster_sync();
+  img_lo = __reduce_min_sync(0xffffffffu, sh.lo[lane & (cluster - 1)]);
+  img_hi = __reduce_max_sync(0xffffffffu, sh.hi[lane & (cluster - 1)]);
 
-  uint64_t bound = ~0ull;  // every element is wanted when there are at most `kept`
-  if (n > kept) {
-    uint64_t prefix = 0, mask = 0;
-    uint32_t rank = static_cast<uint32_t>(kept);  // 1-based rank, among the elements that match `prefix`, of the key wanted
-    for (int pass = 0; pass < 6; ++pass) {
-      const int shift = pass == 0 ? 53 : pass == 1 ? 42 : pass == 2 ? 32 : pass == 3 ? 21 : pass == 4 ? 10 : 0;
-      const uint32_t digit_mask = (pass == 2 || pass == 5) ? 1023u : 2047u;
-      // (Scores of one sequence are close together, so in the top digits most tokens fall into a few bins;
-      // shared-memory atomics on one address still cost less here than finding a warp's equal digits first with
-      // match.any, which was measured: 2.5 us more per launch.)
-      if (kLevel != 2) {
+  // The wanted key is the `rank_left`-th of those with a value in [lo, hi]; all `taken` keys below are wanted, `run` of
+  // them those of CTA number `warp`. The value is the image or, when there are too many keys of one image, the position
+  // of those that have it.
+  uint32_t lo = img_lo, hi = img_hi, tied = 0;
+  bool by_position = false;
+  uint32_t bound;
+  auto value_of = [&](uint32_t image, uint32_t position) { return by_position ? position : image; };
+  auto below = [&](uint32_t image, uint32_t position) {  // wanted whatever the last range's bins say
+    return by_position ? image < tied || (image == tied && position < lo) : image < lo;
+  };
+  auto up_to_bound = [&](uint32_t image, uint32_t position) {
+    return by_position ? image < tied || (image == tied && position <= bound) : image <= bound;
+  };
+  uint32_t rank_left = static_cast<uint32_t>(kept), taken = 0, run = 0, total;
+  int shift;
+  bool dense;  // bins so full that sorting is the shorter way
+  const uint32_t enough = static_cast<uint32_t>(min(kListKeys, k + max(k >> 1, 128)));
+  for (int pass = 0;; ++pass) {
+    const uint32_t span = hi - lo;
+    shift = max(0, 32 - kBinsLog2 - __clz(static_cast<int>(span)));
+    uint32_t* hist = sh.hist[pass & 1];
+    if (!by_position) {
+      for_each([&](uint32_t image, uint32_t) {
+        if (image - lo <= span) atomicAdd(&hist[(image - lo) >> shift], 1u);
+      });
+    } else {
+      for_each([&](uint32_t image, uint32_t position) {
+        if (image == tied && position - lo <= span) atomicAdd(&hist[(position - lo) >> shift], 1u);
+      });
+    }
+    cluster_sync();
+    if (warp < cluster) {  // the bins of CTA `warp`, four at a time
+      const uint32_t src = ptx::MapToRank(ptx::SmemAddr(hist), warp) + lane * 16;
+      uint32_t v[kBins / 128][4];
 #pragma unroll
-        for (int j = 0; j < kHeldPerThread; ++j) {
-          const int e = tid + j * kSortThreads;
-          if (e < n) {
-            const uint64_t key = held_key(j, e);
-            if ((key & mask) == prefix) atomicAdd(&hist[static_cast<uint32_t>(key >> shift) & digit_mask], 1u);
-          }
-        }
-      }
-      for (int e = tid + kFirstRead; e < n; e += kSortThreads) {
-        const uint64_t key = read_key(e);
-        if ((key & mask) == prefix) atomicAdd(&hist[static_cast<uint32_t>(key >> shift) & digit_mask], 1u);
-      }
-      __syncthreads();
-      // A thread owns a few consecutive bins (and clears them for the next pass); a scan over the threads gives the
-      // elements before its bins: shuffles inside the warp, and every warp adds up the warps before it for itself.
-      uint32_t count[kBinsPerThread], mine = 0;
+      for (int q = 0; q < kBins / 128; ++q) ptx::LdClusterV4(src + q * 512, v[q][0], v[q][1], v[q][2], v[q][3]);
 #pragma unroll
-      for (int i = 0; i < kBinsPerThread; ++i) {
-        count[i] = hist[kBinsPerThread * tid + i];
-        hist[kBinsPerThread * tid + i] = 0;
-        mine += count[i];
+      for (int q = 0; q < kBins / 128; ++q) reinterpret_cast<uint4*>(sh.peers[warp])[32 * q + lane] = make_uint4(v[q][0], v[q][1], v[q][2], v[q][3]);
+      if (lane == 0) sh.below[warp] = run;
+    }
+    if (pass > 0 && tid < kBins) sh.hist[(pass + 1) & 1][tid] = 0;  // (the peers are done with it: they have passed the barrier)
+    __syncthreads();
+    uint32_t mine = 0, earlier = 0, incl = 0;  // of bin `tid`: all keys, those of the CTAs before this one
+    if (tid < kBins) {
+      for (int c = 0; c < cluster; ++c) {
+        const uint32_t v = sh.peers[c][tid];
+        mine += v;
+        earlier += c < rank ? v : 0u;
       }
-      uint32_t incl = mine;
+      incl = mine;
 #pragma unroll
       for (int off = 1; off < 32; off <<= 1) {
         const uint32_t up = __shfl_up_sync(0xffffffffu, incl, off);
         if (lane >= off) incl += up;
       }
-      if (lane == 31) warp_sum[warp] = incl;
-      __syncthreads();
-      uint32_t earlier = lane < warp ? warp_sum[lane] : 0u;
-#pragma unroll
-      for (int off = 16; off > 0; off >>= 1) earlier += __shfl_xor_sync(0xffffffffu, earlier, off);
-      uint32_t before = earlier + incl - mine;
-      if (before < rank && rank <= before + mine) {  // one thread: the rank falls in its bins
-#pragma unroll
-        for (int i = 0; i < kBinsPerThread; ++i) {
-          if (before < rank && rank <= before + count[i]) {
-            chosen[pass & 1][0] = kBinsPerThread * tid + i;
-            chosen[pass & 1][1] = before;
-            chosen[pass & 1][2] = count[i];
-          }
-          before += count[i];
-        }
-      }
-      __syncthreads();
-      prefix |= static_cast<uint64_t>(chosen[pass & 1][0]) << shift;
-      mask |= static_cast<uint64_t>(digit_mask) << shift;
-      rank -= chosen[pass & 1][1];
-      bound = prefix;  // after the last pass the prefix is the key itself
-      if (rank == chosen[pass & 1][2]) {  // all that still match are wanted: the bound is the largest key with this prefix
-        bound = prefix | ~mask;
-        break;
-      }
-    }
-  }
-  // Exactly `kept` keys are at most the bound. A warp reserves the slots of its takers with one addition.
-  auto take = [&](bool wanted, uint64_t key) {  // every lane of the warp calls
-    const unsigned takers = __ballot_sync(0xffffffffu, wanted);
-    if (takers == 0u) return;
-    uint32_t slot0 = 0;
-    if (lane == __ffs(takers) - 1) slot0 = atomicAdd(&n_taken, static_cast<uint32_t>(__popc(takers)));
-    slot0 = __shfl_sync(0xffffffffu, slot0, __ffs(takers) - 1);
-    const uint32_t slot = slot0 + __popc(takers & ((1u << lane) - 1u));
-    if (wanted && slot < static_cast<uint32_t>(kMaxK)) keys[slot] = key;
-  };
-  if (kLevel != 2) {
-#pragma unroll
-    for (int j = 0; j < kHeldPerThread; ++j) {
-      const int e = tid + j * kSortThreads;
-      if (warp * 32 + j * kSortThreads >= n) break;
-      const uint64_t key = held_key(j, e);
-      take(e < n && key <= bound, key);
-    }
-  }
-  for (int e0 = warp * 32 + kFirstRead; e0 < n; e0 += kSortThreads) {
-    const int e = e0 + lane;
-    const uint64_t key = e < n ? read_key(e) : ~0ull;
-    take(e < n && key <= bound, key);
-  }
-  __syncthreads();
-  if (kLevel == 1) {  // the chunk's best, in any order: the next level selects and sorts
-    for (int i = tid; i < kept; i += kSortThreads) cand_out[i] = keys[i];
-    return;
-  }
-  // The collected keys in order: a bitonic sort, ascending, of the list padded to a power of two. Element e
-  // belongs to thread e % 1024 (two elements a thread when k > 1024). Steps whose partner is less than 32 away
-  // stay inside a warp and run on registers with shuffles, a whole run of them between two barriers; only the
-  // steps with a partner 32 or more away (10 of the 45 for 512 keys) go through shared memory.
-  int padded = 32;
-  while (padded < kept) padded <<= 1;
-  for (int i = kept + tid; i < padded; i += kSortThreads) keys[i] = ~0ull;
-  __syncthreads();
-  for (int size = 2; size <= padded; size <<= 1) {
-    int stride = size >> 1;
-    for (; stride >= 32; stride >>= 1) {
-      for (int i = tid; i < padded / 2; i += kSortThreads) {
-        const int lo = 2 * i - (i & (stride - 1));  // index of the pair's lower element
-        const int hi = lo + stride;
-        const bool ascending = (lo & size) == 0;
-        const uint64_t a = keys[lo], c = keys[hi];
-        if ((a > c) == ascending) {
-          keys[lo] = c;
-          keys[hi] = a;
-        }
-      }
-      __syncthreads();
-    }
-    for (int e = tid; e < padded; e += kSortThreads) {  // the same trip count for every lane of a warp
-      uint64_t mine = keys[e];
-      const bool ascending = (e & size) == 0;
-      for (int s2 = stride; s2 > 0; s2 >>= 1) {
-        const uint64_t other = __shfl_xor_sync(0xffffffffu, mine, s2);
-        const bool lower = (e & s2) == 0;  // this element is the pair's lower one
-        const bool take_other = lower ? ((mine > other) == ascending) : ((other > mine) == ascending);
-        if (take_other) mine = other;
-      }
-      keys[e] = mine;
+      if (lane == 31) sh.warp_a[warp] = incl;
     }
     __syncthreads();
+    if (tid < kBins) {
+      uint32_t before = incl - mine;
+      for (int w = 0; w < warp; ++w) before += sh.warp_a[w];
+      if (tid == 0) sh.start[0] = taken;
+      sh.start[tid + 1] = taken + before + mine;
+      sh.next[tid] = taken + before + earlier;
+      if (before < rank_left && rank_left <= before + mine) {  // one thread
+        sh.chosen[0] = tid;
+        sh.chosen[1] = before;
+        sh.chosen[2] = mine;
+      }
+      // The comparisons that ordering bin by bin would take: a bin's size squared. (Whatever lies beyond the chosen bin
+      // counts as nothing: it starts at or after the wanted rank.)
+      const uint32_t squares = __reduce_add_sync(0xffffffffu, before < rank_left ? mine * min(mine, 8192u) : 0u);
+      if (lane == 0) sh.warp_b[warp] = squares;
+    }
+    __syncthreads();
+    const uint32_t bin = sh.chosen[0], before = sh.chosen[1], in_bin = sh.chosen[2];
+    const uint32_t offset = (bin << shift) | ((1u << shift) - 1);
+    bound = offset >= span ? hi : lo + offset;
+    total = taken + before + in_bin;
+    if (total <= enough) {  // (a bin of one position holds one key: the passes end)
+      uint32_t squares = taken * taken;
+      for (int w = 0; w < kBins / 32; ++w) squares += sh.warp_b[w];
+      dense = squares > (kMostComparisons << cluster_log2);
+      break;
+    }
+    if (warp < cluster) {
+      uint32_t sum = 0;
+      for (uint32_t t = lane; t < bin; t += 32) sum += sh.peers[warp][t];
+      run += __reduce_add_sync(0xffffffffu, sum);
+    }
+    taken += before;
+    rank_left -= before;
+    lo += bin << shift;
+    hi = bound;
+    if (shift == 0) {  // too many keys of one image
+      by_position = true;
+      tied = lo;
+      lo = 0;
+      hi = static_cast<uint32_t>(len) - 1;
+    }
   }
-  for (int i = tid; i < kept; i += kSortThreads) {
-    const int32_t t = static_cast<int32_t>(keys[i] & 0xffffffffu);
-    p.index[b * k + i] = t;
+  if (tid == 0) {
+    uint32_t at = 0;
+    for (int c = 0; c < rank; ++c) at += sh.below[c];
+    sh.next[kBins] = at;
+  }
+  __syncthreads();
+
+  auto bin_of = [&](uint32_t image, uint32_t position) {  // a key's bin in the list: its first entry and the one after its last
+    if (below(image, position)) return make_uint2(0u, taken);
+    const uint32_t bin = (value_of(image, position) - lo) >> shift;
+    return make_uint2(sh.start[bin], sh.start[bin + 1]);
+  };
+  for_each([&](uint32_t image, uint32_t position) {
+    if (!up_to_bound(image, position)) return;
+    const uint32_t bin = below(image, position) ? static_cast<uint32_t>(kBins) : (value_of(image, position) - lo) >> shift;
+    const uint32_t at = atomicAdd(&sh.next[bin], 1u);
+    const uint64_t key = (static_cast<uint64_t>(image) << 32) | position;
+    if (cluster == 1) {
+      sh.all[at] = key;
+    } else {  // written to the lists below, where the stores are shared out
+      const uint32_t i = atomicAdd(&sh.n_mine, 1u);
+      sh.scratch[i] = key;
+      sh.place[i] = static_cast<uint16_t>(at);
+    }
+  });
+  if (cluster > 1) {
+    __syncthreads();
+    // A key goes to the CTAs whose entries of the list its bin overlaps (to the one that sorts, if sorting it is).
+    const int items = static_cast<int>(sh.n_mine) << cluster_log2;
+    for (int item = tid; item < items; item += kSortThreads) {
+      const int i = item >> cluster_log2, c = item & (cluster - 1);
+      const uint64_t key = sh.scratch[i];
+      const uint2 bin = bin_of(static_cast<uint32_t>(key >> 32), static_cast<uint32_t>(key));
+      const bool theirs = dense ? c == 0 : (total * c) >> cluster_log2 < bin.y && (total * (c + 1)) >> cluster_log2 > bin.x;
+      if (theirs) ptx::StClusterB64(ptx::MapToRank(ptx::SmemAddr(&sh.all[sh.place[i]]), c), key);
+    }
+  }
+  cluster_sync();
+
+  auto write = [&](uint64_t key, int place) {
+    const int32_t t = static_cast<int32_t>(key & 0xffffffffu);
+    p.index[b * k + place] = t;
     if (p.rows_out != nullptr) {  // the selection as pool rows, what ResolveRowsKernel would make of it
       const int64_t column = t / p.block_size;
       const int64_t block = column < p.max_blocks ? p.block_table[static_cast<int64_t>(b) * p.max_blocks + column] : -1;
       const int64_t r = block * p.block_size + t % p.block_size;
       int32_t out_row = -1;
       if (block < 0 || r >= p.pool_rows) {
-        RecordError(p.status, B200KV_DEV_BAD_BLOCK, b, i, t);
+        RecordError(p.status, B200KV_DEV_BAD_BLOCK, b, place, t);
       } else {
         out_row = static_cast<int32_t>(r);
       }
-      p.rows_out[b * k + i] = out_row;
+      p.rows_out[b * k + place] = out_row;
+    }
+  };
+  const int keys = static_cast<int>(total);
+  if (!dense) {
+    // This CTA's entries of the list, `team` neighbouring threads to each.
+    const int entry_lo = (keys * rank) >> cluster_log2, entry_hi = (keys * (rank + 1)) >> cluster_log2;
+    int team_log2 = 0;
+    while (team_log2 < 5 && (entry_hi - entry_lo) << (team_log2 + 1) <= kSortThreads) ++team_log2;
+    const int member = tid & ((1 << team_log2) - 1);
+    for (int e0 = entry_lo; e0 < entry_hi; e0 += kSortThreads >> team_log2) {  // the same trip count for all threads
+      const int entry = e0 + (tid >> team_log2);
+      const bool live = entry < entry_hi;
+      uint64_t key = 0;
+      int begin = 0, end = 0;
+      if (live) {
+        key = sh.all[entry];
+        const uint2 bin = bin_of(static_cast<uint32_t>(key >> 32), static_cast<uint32_t>(key));
+        begin = static_cast<int>(bin.x);
+        end = static_cast<int>(bin.y);
+      }
+      int place = 0;
+#pragma unroll 4
+      for (int i = begin + member; i < end; i += 1 << team_log2) place += sh.all[i] < key ? 1 : 0;
+      for (int off = 1; off < 1 << team_log2; off <<= 1) place += __shfl_xor_sync(0xffffffffu, place, off);
+      place += begin;
+      if (live && member == 0 && place < kept) write(key, place);
+    }
+    return;
+  }
+  if (rank != 0) return;
+  int padded = 32;
+  while (padded < keys) padded <<= 1;
+  for (int i = keys + tid; i < padded; i += kSortThreads) sh.all[i] = ~0ull;
+  __syncthreads();
+  const int threads = min(padded, kSortThreads);
+  if (tid < threads) {
+    if (padded <= kSortThreads) {
+      SortKeys<1>(sh.all, sh.scratch, threads);
+    } else if (padded == 2 * kSortThreads) {
+      SortKeys<2>(sh.all, sh.scratch, threads);
+    } else {
+      SortKeys<4>(sh.all, sh.scratch, threads);
     }
   }
+  __syncthreads();
+  for (int i = tid; i < kept; i += kSortThreads) write(sh.all[i], i);
+}
+
+int32_t LaunchSelect(const SelectParams& p, int32_t batch, int64_t max_kv_len, cudaStream_t stream) {
+  // How many clusters of 1, 2, 4, 8, 16 CTAs the device holds at once; looked up once per thread and device.
+  static thread_local int known_device = -1;
+  static thread_local int32_t most[5];
+  int device = 0;
+  if (int32_t rc = CheckCuda(cudaGetDevice(&device), "cudaGetDevice")) return rc;
+  cudaLaunchConfig_t config = {};
+  config.blockDim = dim3(kSortThreads);
+  config.dynamicSmemBytes = sizeof(SelectShared);
+  config.stream = stream;
+  cudaLaunchAttribute attrs[2];
+  attrs[0].id = cudaLaunchAttributeClusterDimension;
+  attrs[0].val.clusterDim.y = 1;
+  attrs[0].val.clusterDim.z = 1;
+  attrs[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attrs[1].val.programmaticStreamSerializationAllowed = 1;
+  config.attrs = attrs;
+  if (device != known_device) {
+    if (int32_t rc = CheckCuda(cudaFuncSetAttribute(IndexerSelectKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(SelectShared))), "indexer top-k smem opt-in")) return rc;
+    if (int32_t rc = CheckCuda(cudaFuncSetAttribute(IndexerSelectKernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1), "indexer top-k cluster opt-in")) return rc;
+    for (int i = 0; i < 5; ++i) {
+      attrs[0].val.clusterDim.x = 1u << i;
+      config.gridDim = dim3(1u << i);
+      config.numAttrs = 1;
+      int clusters = 0;
+      if (cudaOccupancyMaxActiveClusters(&clusters, IndexerSelectKernel, &config) != cudaSuccess) {
+        cudaGetLastError();  // a size the device does not offer
+        clusters = 0;
+      }
+      most[i] = clusters;
+    }
+    known_device = device;
+  }
+  int size = 0;
+  while (size < 4 && max_kv_len > static_cast<int64_t>(kTokensPerCta) << size) ++size;
+  while (size > 0 && batch > most[size]) --size;
+  attrs[0].val.clusterDim.x = 1u << size;
+  config.gridDim = dim3(1u << size, static_cast<unsigned>(batch));
+  config.numAttrs = 2;
+  return CheckCuda(cudaLaunchKernelEx(&config, IndexerSelectKernel, p), "indexer top-k launch");
 }
 
 }  // namespace
@@ -383,9 +581,11 @@ int32_t LaunchIndexerScoreTc(const void* q, const float* q_scale, const void* we
 using namespace b200kv;
 
 namespace {
-// Scores [batch][stride] fp32, then (sequences longer than one chunk) the candidate keys [batch][chunks][kMaxK].
+// Scores [batch][stride] fp32. Sequences of more than 8,192 tokens have always asked for room for 2,048 keys a chunk of
+// that length behind the scores; the selection no longer needs it, callers' plans are sized by it.
+constexpr int64_t kPlanChunk = 8192;
 int64_t ScoreStrideOf(int64_t max_kv_len) { return (max_kv_len + 3) & ~3ll; }
-int64_t ChunksOf(int64_t max_kv_len) { return (max_kv_len + kSelectChunk - 1) / kSelectChunk; }
+int64_t ChunksOf(int64_t max_kv_len) { return (max_kv_len + kPlanChunk - 1) / kPlanChunk; }
 size_t ScoreBytesOf(int32_t batch, int64_t max_kv_len) {
   return (static_cast<size_t>(batch) * static_cast<size_t>(ScoreStrideOf(max_kv_len)) * sizeof(float) + 15) & ~static_cast<size_t>(15);
 }
@@ -467,8 +667,6 @@ extern "C" int32_t b200kv_indexer_topk(const b200kv_indexer_args* args, void* st
   sp.score_stride = p.score_stride;
   sp.kv_len = a.kv_len;
   sp.k = a.k;
-  sp.chunks = static_cast<int32_t>(ChunksOf(a.max_kv_len));
-  sp.candidates = reinterpret_cast<uint64_t*>(static_cast<char*>(a.workspace) + ScoreBytesOf(a.batch, a.max_kv_len));
   sp.index = a.index_out;
   sp.n_selected = a.n_selected_out;
   sp.block_table = a.block_table;
@@ -477,15 +675,5 @@ extern "C" int32_t b200kv_indexer_topk(const b200kv_indexer_args* args, void* st
   sp.pool_rows = a.pool_rows;
   sp.rows_out = a.rows_out;
   sp.status = static_cast<int32_t*>(status);
-  if (sp.chunks <= 1) {
-    return CheckCuda(LaunchOverlapped(IndexerSelectKernel<0>, dim3(static_cast<unsigned>(a.batch)), dim3(kSortThreads), 0, s, sp),
-                     "indexer top-k launch");
-  }
-  if (int32_t rc = CheckCuda(LaunchOverlapped(IndexerSelectKernel<1>, dim3(static_cast<unsigned>(sp.chunks), static_cast<unsigned>(a.batch)),
-                                              dim3(kSortThreads), 0, s, sp),
-                             "indexer top-k (chunks) launch")) {
-    return rc;
-  }
-  return CheckCuda(LaunchOverlapped(IndexerSelectKernel<2>, dim3(static_cast<unsigned>(a.batch)), dim3(kSortThreads), 0, s, sp),
-                   "indexer top-k (candidates) launch");
+  return LaunchSelect(sp, a.batch, a.max_kv_len, s);
 }

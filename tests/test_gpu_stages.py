@@ -259,6 +259,35 @@ def test_indexer_selection_matches_oracle_bit_for_bit(lens, k):
     assert np.array_equal(index.cpu().numpy(), exp_index), "selection differs from the oracle"
 
 
+@pytest.mark.parametrize("length", [500, 4096, 5000, 20000, 70000, 150000])
+@pytest.mark.parametrize("shape", ["equal", "outlier", "two values"])
+def test_indexer_selection_of_scores_that_bins_do_not_separate(length, shape):
+    """All scores equal (positions decide, in passes down to single positions), one score a million times the others
+    (the first histogram sees one filled bin), and two values; every cluster size (one CTA per 4,096 tokens up to 16)
+    and more tokens than a CTA holds in registers. A token's score is its key scale: one head, q = k = one-hot."""
+    bs, k = 64, 300
+    blocks = (length + bs - 1) // bs
+    q = torch.zeros((1, 1, 128), dtype=torch.uint8, device="cuda")
+    q[..., 0] = 0x38  # 1.0
+    key = torch.zeros((blocks * bs, 128), dtype=torch.uint8, device="cuda")
+    key[:, 0] = 0x38
+    g = torch.Generator(device="cuda")
+    g.manual_seed(length)
+    ks = torch.full((blocks * bs,), 0.5, device="cuda")
+    if shape == "outlier":
+        ks = 0.5 + 0.001 * torch.rand((blocks * bs,), generator=g, device="cuda")
+        ks[length // 3] = 5e5
+    elif shape == "two values":
+        ks[torch.rand((blocks * bs,), generator=g, device="cuda") < 200.0 / length] = 0.75
+    one = torch.ones((1, 1), device="cuda")
+    table = torch.arange(blocks, device="cuda", dtype=torch.int32)[None]
+    index, n = b200kv.indexer_topk(q, one, one.bfloat16(), key, ks, table, to_dev_i32([length]), bs, length, k,
+                                   variant=b200kv.INDEXER_EXACT)
+    want = torch.sort(ks[:length].cpu(), descending=True, stable=True).indices[:k]
+    assert int(n[0]) == min(k, length)
+    assert torch.equal(index[0].cpu().long(), want)
+
+
 def _check_selection_up_to_rounding(index, n_sel, got_scores, exp_scores, exp_n, kv_len, k, eps_rel):
     """The tensor-core scores differ from the oracle's by rounding, so its selection is checked as a selection:
     per sequence the count, positions distinct and inside the sequence, the device's own scores in best-first
