@@ -33,7 +33,8 @@
 // 91 KB that a CTA takes in, 0.6 softmax, 0.7 PV, 0.6 + 0.9 exchange, 1.0 merge; 16 sequences of 300 .. 4,096 tokens in
 // pages of 16 rows 360 (CUDA-core kernel) -> 53.6; 32 sequences of up to 2,048 tokens with 16 heads 373 -> 25.4.
 //
-// Roles as in the flat kernel: warps 0-3 softmax and epilogue, 4 producer, 5 QK, 6 PV. Every wait is bounded; a CTA
+// Roles as in the flat kernel: warps 0-3 softmax, 4 producer, 5 QK, 6 PV; all eight warps take part in the exchange and
+// the merge. Every wait is bounded; a CTA
 // that gives up still arrives at the cluster barriers, so no peer is left waiting.
 #include <cuda.h>
 #include <cuda_fp8.h>
@@ -53,7 +54,7 @@ namespace {
 
 using namespace mla;
 
-constexpr int kThreads = 224;
+constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
 constexpr int kMaxCluster = 16;
 constexpr int kDvGroup = 32;     // a warp's share of an accumulator: the unit in which columns change hands
@@ -142,7 +143,10 @@ struct Share {
 
 __device__ __forceinline__ Share ShareOf(int tiles, int cluster, int rank, int group_heads) {
   int log2 = 31 - __clz(cluster), heads = group_heads;
-  while (heads > kLeastHeads && log2 > 0 && 2 * tiles <= (1 << log2)) {
+  // Halving the ranges halves what a CTA sends (64 KB at 64 heads and some 30 bytes a cycle) and the heads of Q it loads,
+  // and adds tiles (72 KB at 27 bytes a cycle): worth it while it adds none, and from 64 heads also for the second tile
+  // of some CTAs (one sequence of 1,024 tokens: 16.1 us in 16 ranges, 12.9 us in 8).
+  while (heads > kLeastHeads && log2 > 0 && (2 * tiles <= (1 << log2) || (heads == kHeads && 2 * tiles <= (3 << log2)))) {
     --log2;
     heads >>= 1;
   }
@@ -286,7 +290,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
       }
     } else if constexpr (kSource == kTiles) {
-      for (int c = 3 * (warp - 4); c < 3 * (warp - 4) + 3; ++c) issue_slab(first_row, 0, c);
+      for (int c = 3 * (warp - 4); c < min(3 * (warp - 4) + 3, 9); ++c) issue_slab(first_row, 0, c);
     }
     if (warp == 4 && appends) {  // the sequence's new row, towards shared memory
       const uint32_t full = bar(&misc->new_row_full);
@@ -728,66 +732,159 @@ __global__ void __launch_bounds__(kThreads, 1)
 
   // ======================= exchange and merge =====================================================
   const bool direct = TilesOf(len) <= share.ranges && share.heads <= 32;  // the same in all CTAs of the cluster
+  const int columns_log2 = 9 - share.ranges_log2;  // this CTA merges 512 / S output columns: range * columns ..
+  const int columns = 1 << columns_log2;
+  const int quads = share.heads >> 2;
+  const int first = head_first + share.head_lo;
+  const bool want_partial = p.user_o != nullptr;
+  // Four heads of one output column: lane = column, so an output store of the warp is 64 contiguous bytes of a row.
+  auto emit = [&](int quad, int dv, const float (&acc)[4]) {  // every lane of the warp calls
+    const int64_t row0 = static_cast<int64_t>(seq) * p.heads + first + 4 * quad;
+    const int valid = p.heads - first - 4 * quad;  // heads of the quad that exist: four or more but for an odd count's last
+    if (want_partial) {
+      float* dst = p.user_o + row0 * kLatent + dv;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        if (i < valid) dst[i * kLatent] = acc[i];
+      }
+      return;
+    }
+    __nv_bfloat16 y[4];
+    __nv_bfloat16* dst = p.out + row0 * kLatent + dv;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      y[i] = __float2bfloat16_rn(acc[i]);
+      if (i < valid) dst[i * kLatent] = y[i];
+    }
+    if (p.out_q != nullptr) {  // (64 heads: every quad is whole)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        // The 32 columns of a row that a warp holds are one MX block, as in the flat kernel's merge.
+        const float x = __bfloat162float(y[i]);
+        const uint32_t top = __reduce_max_sync(0xffffffffu, __float_as_uint(x) & 0x7fffffffu);
+        const bool nan = top > 0x7f800000u;
+        const MxScale block = MxScaleOf(__uint_as_float(top), nan);
+        const uint32_t code = nan ? (((__float_as_uint(x) >> 24) & 0x80u) | 0x7fu)
+                                  : static_cast<uint32_t>(__nv_cvt_float_to_fp8(__fmul_rn(x, block.inv), __NV_SATFINITE, __NV_E4M3));
+        p.out_q[(row0 + i) * kLatent + dv] = static_cast<uint8_t>(code);
+        if (lane == 0) p.out_scale[(row0 + i) * (kLatent / 32) + (dv >> 5)] = static_cast<uint8_t>(block.code);
+      }
+    }
+  };
+  auto emit_ml = [&](int h, float big, float total) {  // head h of this CTA's
+    if (first + h >= p.heads) return;
+    const int64_t at = static_cast<int64_t>(seq) * p.heads + first + h;
+    const float m_nat = big * 0.6931471805599453f;
+    if (want_partial) {
+      p.user_m[at] = m_nat;
+      p.user_l[at] = total;
+    } else if (p.lse != nullptr) {
+      p.lse[at] = total > 0.0f ? m_nat + logf(total) : -INFINITY;
+    }
+  };
+  // (m, l) of this CTA's token range: lane j < 16 of a softmax warp takes row j of the warp's sixteen.
+  const int from = 4 * (lane & 7);
+  const float m_lo = __shfl_sync(0xffffffffu, m_run[0], from), m_hi = __shfl_sync(0xffffffffu, m_run[1], from);
+  const float l_lo = __shfl_sync(0xffffffffu, l_run[0], from), l_hi = __shfl_sync(0xffffffffu, l_run[1], from);
+  const bool failed = __any_sync(0xffffffffu, !ok);
+  const float m_row = (lane & 8) ? m_hi : m_lo;
+  const float l_row = failed ? 0.0f : ((lane & 8) ? l_hi : l_lo);
+  const bool has_row = warp < 4 && lane < 16 && warp * 16 < share.heads;
+  const int h_row = warp * 16 + lane;
+  // The accumulators: warp w reads lanes 32 (w % 4) .. of numbers w / 4 and w / 4 + 2.
+  const uint32_t acc_base = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16) + 64 * (warp >> 2);
+  const int dv_warp = 128 * (warp >> 2) + 32 * (warp & 3);  // output column of lane 0 in the first of the two, + 256 in the other
+  if (n > 0 && warp >= 4) WarpSpin(bar(&misc->o_full), 0, misc, p.status, 233);
   ptx::ClusterWait();
+
+  if (share.ranges == 1) {
+    // Nobody to exchange with: out of the accumulators straight into the rows.
+    float* s_norm = reinterpret_cast<float*>(smem + kOffW);
+    if (has_row) {
+      s_norm[h_row] = want_partial ? 1.0f : (l_row > 0.0f ? 1.0f / l_row : 0.0f);
+      emit_ml(h_row, m_row, l_row);
+    }
+    __syncthreads();
+    ptx::TcFenceAfterSync();
+#pragma unroll 1
+    for (int part = 0; part < 4; ++part) {  // 32 heads of one of the two accumulators
+      const int half = part & 1, dv = dv_warp + 256 * (part >> 1) + lane;
+      if (32 * half >= share.heads) continue;
+      uint32_t o[32];
+      ptx::TmemLd32(acc_base + 128 * (part >> 1) + 32 * half, o);
+      ptx::TmemWaitLd();
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const int quad = 8 * half + q;
+        if (quad >= quads || first + 4 * quad >= p.heads) break;
+        const float4 w = *reinterpret_cast<const float4*>(&s_norm[4 * quad]);
+        float acc[4];
+        acc[0] = n > 0 ? __uint_as_float(o[4 * q]) * w.x : 0.0f;
+        acc[1] = n > 0 ? __uint_as_float(o[4 * q + 1]) * w.y : 0.0f;
+        acc[2] = n > 0 ? __uint_as_float(o[4 * q + 2]) * w.z : 0.0f;
+        acc[3] = n > 0 ? __uint_as_float(o[4 * q + 3]) * w.w : 0.0f;
+        emit(quad, dv, acc);
+      }
+    }
+    ptx::TcFenceBeforeSync();
+    __syncthreads();
+    if (warp == 5) {
+      ptx::TcFenceAfterSync();
+      ptx::TmemDealloc(tmem, kTmemCols);
+    }
+    return;
+  }
+
   if (!direct) {
     ptx::ClusterArrive();
     ptx::ClusterWait();  // every CTA is done with its tiles: the KV stages and Q's place of all of them are free
   }
-  const int columns_log2 = 9 - share.ranges_log2;  // this CTA merges 512 / S output columns: range * columns ..
-  const int columns = 1 << columns_log2;
-  const int quads = share.heads >> 2;
+  ptx::TcFenceAfterSync();
   const uint32_t ml_off = direct ? kOffMlDirect : kOffMl;  // m, then l
   const uint32_t mail_off = direct ? kOffKv + kStageBytes : kOffKv;
   const uint32_t mail_mine = base + mail_off + share.range * (columns * share.heads * 4);
-  if (warp < 4) {
-    // (m, l) of this CTA's token range to the CTAs of the same columns; lane j < 16 has row j of the warp's sixteen.
-    const int from = 4 * (lane & 7);
-    const float m_lo = __shfl_sync(0xffffffffu, m_run[0], from), m_hi = __shfl_sync(0xffffffffu, m_run[1], from);
-    const float l_lo = __shfl_sync(0xffffffffu, l_run[0], from), l_hi = __shfl_sync(0xffffffffu, l_run[1], from);
-    const bool failed = __any_sync(0xffffffffu, !ok);
-    if (lane < 16 && warp * 16 < share.heads) {
-      const uint32_t at = static_cast<uint32_t>(share.range * kHeads + warp * 16 + lane) * 4;
-      const float m = (lane & 8) ? m_hi : m_lo;
-      const float l = failed ? 0.0f : ((lane & 8) ? l_hi : l_lo);
+  if (has_row) {
+    const uint32_t at = static_cast<uint32_t>(share.range * kHeads + h_row) * 4;
 #pragma unroll 4
-      for (int s = 0; s < share.ranges; ++s) {
-        const uint32_t dst = ptx::MapToRank(base + ml_off + at, share.first_peer + s);
-        ptx::StClusterF32(dst, m);
-        ptx::StClusterF32(dst + kMlBytes, l);
-      }
+    for (int s = 0; s < share.ranges; ++s) {
+      const uint32_t dst = ptx::MapToRank(base + ml_off + at, share.first_peer + s);
+      ptx::StClusterF32(dst, m_row);
+      ptx::StClusterF32(dst + kMlBytes, l_row);
     }
-    // O^T: a warp's 32 columns of an accumulator lie inside one CTA's share. The mailbox is [range][head quad][columns]
-    // [4 heads] fp32, so a store of the warp is 512 contiguous bytes.
-    if (n > 0 && !failed) {
-      const uint32_t lane_base = static_cast<uint32_t>(warp * 32) << 16;
-      if (share.heads == kLeastHeads) {  // all four accumulators behind one wait
-        uint32_t o[4][16];
+  }
+  // O^T: a warp's 32 columns of an accumulator lie inside one CTA's share. The mailbox is [range][head quad][columns]
+  // [4 heads] fp32, so a store of the warp is 512 contiguous bytes. (A CTA that failed sends l = 0, which makes what it
+  // sends here count for nothing.)
+  if (n > 0) {
+    uint32_t dst[2];
 #pragma unroll
-        for (int tm = 0; tm < 4; ++tm) ptx::TmemLd16(tmem + lane_base + 64 * tm, o[tm]);
-        ptx::TmemWaitLd();
+    for (int a = 0; a < 2; ++a) {
+      const int dv = dv_warp + 256 * a;
+      dst[a] = ptx::MapToRank(mail_mine + ((dv & (columns - 1)) + lane) * 16, static_cast<uint32_t>(share.first_peer + (dv >> columns_log2)));
+    }
+    if (share.heads == kLeastHeads) {
+      uint32_t o[2][16];
+      ptx::TmemLd16(acc_base, o[0]);
+      ptx::TmemLd16(acc_base + 128, o[1]);
+      ptx::TmemWaitLd();
 #pragma unroll
-        for (int tm = 0; tm < 4; ++tm) {
-          const int dv = 128 * tm + 32 * warp;
-          const uint32_t dst = ptx::MapToRank(mail_mine + ((dv & (columns - 1)) + lane) * 16,
-                                              static_cast<uint32_t>(share.first_peer + (dv >> columns_log2)));
+      for (int a = 0; a < 2; ++a) {
 #pragma unroll
-          for (int j = 0; j < 4; ++j) ptx::StClusterV4(dst + j * columns * 16, o[tm][4 * j], o[tm][4 * j + 1], o[tm][4 * j + 2], o[tm][4 * j + 3]);
-        }
+        for (int j = 0; j < 4; ++j) ptx::StClusterV4(dst[a] + j * columns * 16, o[a][4 * j], o[a][4 * j + 1], o[a][4 * j + 2], o[a][4 * j + 3]);
       }
+    } else {
 #pragma unroll 1
-      for (int tm = share.heads == kLeastHeads ? 4 : 0; tm < 4; ++tm) {
-        const int dv = 128 * tm + 32 * warp;
-        const uint32_t dst = ptx::MapToRank(mail_mine + ((dv & (columns - 1)) + lane) * 16,
-                                            static_cast<uint32_t>(share.first_peer + (dv >> columns_log2)));
-        uint32_t lo[32], hi[32];
-        ptx::TmemLd32(tmem + lane_base + 64 * tm, lo);
-        if (share.heads > 32) ptx::TmemLd32(tmem + lane_base + 64 * tm + 32, hi);
+      for (int half = 0; half < share.heads >> 5; ++half) {
+        uint32_t o[2][32];
+        ptx::TmemLd32(acc_base + 32 * half, o[0]);
+        ptx::TmemLd32(acc_base + 128 + 32 * half, o[1]);
         ptx::TmemWaitLd();
 #pragma unroll
-        for (int j = 0; j < 8; ++j) ptx::StClusterV4(dst + j * columns * 16, lo[4 * j], lo[4 * j + 1], lo[4 * j + 2], lo[4 * j + 3]);
-        if (share.heads > 32) {
+        for (int a = 0; a < 2; ++a) {
 #pragma unroll
-          for (int j = 0; j < 8; ++j) ptx::StClusterV4(dst + (8 + j) * columns * 16, hi[4 * j], hi[4 * j + 1], hi[4 * j + 2], hi[4 * j + 3]);
+          for (int j = 0; j < 8; ++j) {
+            ptx::StClusterV4(dst[a] + (8 * half + j) * columns * 16, o[a][4 * j], o[a][4 * j + 1], o[a][4 * j + 2], o[a][4 * j + 3]);
+          }
         }
       }
     }
@@ -801,14 +898,11 @@ __global__ void __launch_bounds__(kThreads, 1)
     ptx::TmemDealloc(tmem, kTmemCols);
   }
 
-  // A unit is 32 columns x 4 heads: lane = column, so an output store of the warp is 64 contiguous bytes of a row. A warp
-  // takes consecutive units, quad after quad, and works a quad's weights out for itself (lane = range x head, the maxima
-  // and sums are shuffles).
+  // A unit is 32 columns x 4 heads. A warp takes consecutive units, quad after quad, and works a quad's weights out for
+  // itself (lane = range x head, the maxima and sums are shuffles).
   const float* s_m = reinterpret_cast<const float*>(smem + ml_off);
   const float* s_l = reinterpret_cast<const float*>(smem + ml_off + kMlBytes);
   float4* s_w = reinterpret_cast<float4*>(smem + kOffW) + warp * kMaxCluster;  // [range] of the warp's present quad
-  const bool want_partial = p.user_o != nullptr;
-  const int first = head_first + share.head_lo;
   const int groups_log2 = columns_log2 - 5;  // columns / 32
   const int units = quads << groups_log2;
   const int unit_lo = units * warp / kWarps, unit_hi = units * (warp + 1) / kWarps;
@@ -845,16 +939,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         const int s = (lane >> 2) + 8 * k;
         if (s < share.ranges) reinterpret_cast<float*>(s_w)[4 * s + (lane & 3)] = m[k] * norm;
       }
-      if (share.range == 0 && lane < 4 && (unit & ((1 << groups_log2) - 1)) == 0 && first + h < p.heads) {
-        const int64_t at = static_cast<int64_t>(seq) * p.heads + first + h;
-        const float m_nat = big * 0.6931471805599453f;
-        if (want_partial) {
-          p.user_m[at] = m_nat;
-          p.user_l[at] = total;
-        } else if (p.lse != nullptr) {
-          p.lse[at] = total > 0.0f ? m_nat + logf(total) : -INFINITY;
-        }
-      }
+      if (share.range == 0 && lane < 4 && (unit & ((1 << groups_log2) - 1)) == 0) emit_ml(h, big, total);
       __syncwarp();
     }
     float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
@@ -868,38 +953,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       acc[2] = fmaf(w.z != 0.0f ? v.z : 0.0f, w.z, acc[2]);
       acc[3] = fmaf(w.w != 0.0f ? v.w : 0.0f, w.w, acc[3]);
     }
-    const int dv = (share.range << columns_log2) + local;
-    const int64_t row0 = static_cast<int64_t>(seq) * p.heads + first + 4 * quad;
-    const int valid = p.heads - first - 4 * quad;  // heads of the quad that exist: four or more but for an odd count's last
-    if (want_partial) {
-      float* dst = p.user_o + row0 * kLatent + dv;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        if (i < valid) dst[i * kLatent] = acc[i];
-      }
-      continue;
-    }
-    __nv_bfloat16 y[4];
-    __nv_bfloat16* dst = p.out + row0 * kLatent + dv;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      y[i] = __float2bfloat16_rn(acc[i]);
-      if (i < valid) dst[i * kLatent] = y[i];
-    }
-    if (p.out_q != nullptr) {  // (64 heads: every quad is whole)
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        // The 32 columns of a row that a warp holds are one MX block, as in the flat kernel's merge.
-        const float x = __bfloat162float(y[i]);
-        const uint32_t top = __reduce_max_sync(0xffffffffu, __float_as_uint(x) & 0x7fffffffu);
-        const bool nan = top > 0x7f800000u;
-        const MxScale block = MxScaleOf(__uint_as_float(top), nan);
-        const uint32_t code = nan ? (((__float_as_uint(x) >> 24) & 0x80u) | 0x7fu)
-                                  : static_cast<uint32_t>(__nv_cvt_float_to_fp8(__fmul_rn(x, block.inv), __NV_SATFINITE, __NV_E4M3));
-        p.out_q[(row0 + i) * kLatent + dv] = static_cast<uint8_t>(code);
-        if (lane == 0) p.out_scale[(row0 + i) * (kLatent / 32) + (dv >> 5)] = static_cast<uint8_t>(block.code);
-      }
-    }
+    emit(quad, (share.range << columns_log2) + local, acc);
   }
 }
 
@@ -1038,6 +1092,26 @@ int32_t Launch(const b200kv_decode_args& a, int source, bool split_p, int32_t cl
 
 }  // namespace
 
+// Up to how many tiles in its longest sequence a batch is better off here than in the flat kernel, which spreads all
+// tiles over all SMs but pays for two launches and the merge of every sequence's parts. Both sides measured (us a layer,
+// flat -> here, all sequences of the length / lengths from a sixteenth of it):
+//   16 CTAs  1 x 2,048: 16.3 -> 16.4, 1 x 4,096: 16.5 -> 19.9; 2 x 4,096: 22.1 -> 20.3, 4 x 4,096: 25.2 -> 20.9 / 24.4 -> 18.9
+//            (three or four sequences of many parts are the merge kernel's worst case); 8 x 2,048: 21.3 -> 19.9, 8 x 4,096:
+//            25.1 -> 27.3
+//    8 CTAs  16 x 1,024: 21.4 -> 19.5 / 20.6 -> 19.2, 16 x 2,048: 25.1 -> 26.7
+//    4 CTAs  32 x 1,024: 23.2 -> 21.8 / 21.1 -> 20.7, 32 x 4,096: 45.2 -> 44.9 / 33.8 -> 42.6
+//    2 CTAs  64 x 512: 27.9 -> 22.5 / 24.2 -> 22.0, 64 x 1,024: 34.8 -> 30.5
+//    1 CTA   128 x 512: 42.1 -> 29.2; 140 x 512: / 38.2 -> 31.5; 128 x 1,024: 56.9 -> 44.8
+int64_t MostTilesFor(int32_t cluster, int32_t batch) {
+  switch (cluster) {
+    case 16: return batch >= 2 && batch <= 4 ? 64 : 32;
+    case 8: return 16;
+    case 4: return 16;
+    case 2: return 12;
+    default: return 8;
+  }
+}
+
 // Work small enough for the cluster kernel: *launched says whether the call was taken. The caller has checked that the
 // flat kernel could take it.
 int32_t TryDecodeCluster(const b200kv_decode_args& a, cudaStream_t stream, int32_t* status, bool* launched) {
@@ -1047,15 +1121,10 @@ int32_t TryDecodeCluster(const b200kv_decode_args& a, cudaStream_t stream, int32
   const ClusterLimits* limits = nullptr;
   if (int32_t rc = LimitsOf(&limits)) return rc;
   const int32_t cluster = ClusterSizeFor(*limits, a.batch);
-  // The flat kernel costs some 19 us + 1.75 us a tile per SM; this one some 8 us + 1.75 us a tile of its longest CTA. It
-  // spreads one sequence over its own cluster only, so where lengths differ much it can need up to C / 148 of the flat
-  // kernel's SMs for the longest; eight tiles per CTA keep it ahead of the flat kernel even when all tiles are in one
-  // sequence (8 + 14 us against 19 + 1.75 ..), and further ahead the fewer there are.
-  // The lengths are on the device; the table (or row list) says how long a sequence can be at most.
+  // The lengths are on the device; the table (or row list) says how many tiles a sequence can have at most.
   const int64_t most_tiles = a.row_index != nullptr ? (a.row_index_stride + kTile - 1) / kTile
                                                     : a.max_blocks * ((a.block_size + kTile - 1) / kTile);
-  constexpr int64_t kMostTilesPerCta = 8;
-  if (a.batch > limits->most[0] || most_tiles > kMostTilesPerCta * cluster) return B200KV_OK;
+  if (most_tiles > MostTilesFor(cluster, a.batch)) return B200KV_OK;
   *launched = true;
   return Launch(a, a.row_index != nullptr ? kRowList : kTiles, false, cluster, kHeads, stream, status);
 }
