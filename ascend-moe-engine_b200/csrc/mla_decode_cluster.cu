@@ -13,20 +13,12 @@
 // tile, because the second stage is then free from the start), and one after it.
 //
 // With a tile or two per CTA everything is latency, so the code between the waits is kept short: shifts for divisions
-// (S, H and C are powers of two), waits that spin instead of parking (a parked thread resumes some 500 cycles late, and
-// nobody else needs the issue slots), loads issued from all warps at once.
+// (S, H and C are powers of two), loads issued from all warps at once.
 //
-// Where the tiles come from (kSource): tiles of 64 rows by TMA through the block table (block sizes that are multiples
-// of 64); the same in boxes of 8, 16 or 32 rows (block sizes that are multiples of those); rows of a caller's list, or
-// rows through a block table with blocks of any size, the latter two with 16-byte asynchronous copies placed as the
-// swizzled TMA load would place them.
-//
-// kSplitP: the softmax weights go to the tensor cores as two bf16 terms (P = hi + lo, 16 bits of it) instead of one,
-// for the geometries whose other kernel keeps them in fp32 (any page size, any head count): twice the PV instructions
-// for an error of 2^-17 of a weight, which the bf16 result does not show. The tensor core truncates its fp32 running sum
-// after every K = 16 step, 36 of them for a score, a bias that the log-sum-exp keeps (5e-7 of it, where fp32 fmas are off
-// by 1.7e-7); so here each slab group of Q.K has an accumulator of its own (8 to 12 steps) and the four are added in
-// fp32, at the price of S being single-buffered.
+// With many tiles a stage's round trip bounds the loop, some 3,500 cycles a tile with the two stages in turn (stamps):
+// 2,200 to a load's last byte, 250 to the softmax's wake-up, 1,100 of softmax, 1,900 until PV, which shares the tensor pipe
+// with the next tile's QK, gives the last slab group back. (QK holding back while a PV is due was 20 % slower; waits that
+// spin instead of parking 1 %.)
 //
 // Measured (B200, graph of layers, us a layer): one sequence of 129 tokens with the append 16.4 (flat kernel and merge)
 // -> 7.9, of which 0.9 from the previous layer's end to the wait's return, 0.4 issue, 1.1 latency, 1.1 QK behind the
@@ -163,10 +155,11 @@ __device__ __forceinline__ Share ShareOf(int tiles, int cluster, int rank, int g
   return s;
 }
 
-// A bounded wait that spins, by all lanes of a warp together.
-__device__ __forceinline__ bool WarpSpin(uint32_t bar, uint32_t parity, Misc* misc, int32_t* status, int site) {
+// A bounded wait by all lanes of a warp together. A phase that is complete already, the usual case for a tile's later slab
+// groups, costs a probe and no call.
+__device__ __forceinline__ bool WarpWait(uint32_t bar, uint32_t parity, Misc* misc, int32_t* status, int site) {
   if (__all_sync(0xffffffffu, ptx::MbarTestWait(bar, parity))) return true;
-  return __all_sync(0xffffffffu, BoundedSpin(bar, parity, misc, status, site));
+  return __all_sync(0xffffffffu, BoundedWait(bar, parity, misc, status, site));
 }
 
 template <int kSource, bool kSplitP>
@@ -355,7 +348,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll 1
         for (int c = 0; c < kGroups && ok; ++c) {
           if (i >= kStages) {
-            ok = WarpSpin(bar(&misc->kv_empty[stage][c]), ((i / kStages) & 1) ^ 1, misc, p.status, 210);
+            ok = WarpWait(bar(&misc->kv_empty[stage][c]), ((i / kStages) & 1) ^ 1, misc, p.status, 210);
             if (!ok) break;
           }
 #pragma unroll 1
@@ -464,9 +457,9 @@ __global__ void __launch_bounds__(kThreads, 1)
         const int64_t row = share.head_lo == 0 ? tile_row_checked(begin, share.t_hi - 1) : -1;
         const int4* src = reinterpret_cast<const int4*>(misc->new_row);
         unsigned char* tile = smem + kOffKv + (last % kStages) * kStageBytes;
-        ok = WarpSpin(bar(&misc->new_row_full), 0, misc, p.status, 212);
+        ok = WarpWait(bar(&misc->new_row_full), 0, misc, p.status, 212);
         for (int g = 0; g < kGroups && ok; ++g) {
-          ok = WarpSpin(bar(&misc->kv_full[last % kStages][g]), (last / kStages) & 1, misc, p.status, 213);
+          ok = WarpWait(bar(&misc->kv_full[last % kStages][g]), (last / kStages) & 1, misc, p.status, 213);
           if (!ok) break;
           const int c = 16 * g + lane;  // 16-byte chunks: eight to a slab's 128-byte row
           if (lane < (g == kGroups - 1 ? 24 : 16)) {
@@ -510,14 +503,14 @@ __global__ void __launch_bounds__(kThreads, 1)
       const uint32_t d = tmem_u + kTmemColS + kTile * buf;
       constexpr uint32_t kNext = kSplitP ? kTile : 0;  // kSplitP: an accumulator per slab group
       auto group_ready = [&](int c) {
-        ok = WarpSpin(bar(&misc->kv_full[stage][c]), kv_parity, misc, p.status, 224 + c);
-        if (ok && i == 0) ok = WarpSpin(bar(&misc->q_full[c]), 0, misc, p.status, 222);
-        if (ok && appends && i == n_u - 1) ok = WarpSpin(bar(&misc->patched[c]), 0, misc, p.status, 223);
+        ok = WarpWait(bar(&misc->kv_full[stage][c]), kv_parity, misc, p.status, 224 + c);
+        if (ok && i == 0) ok = WarpWait(bar(&misc->q_full[c]), 0, misc, p.status, 222);
+        if (ok && appends && i == n_u - 1) ok = WarpWait(bar(&misc->patched[c]), 0, misc, p.status, 223);
         if (!ok) return;
         ptx::TcFenceAfterSync();
         if constexpr (kCopied) ptx::FenceProxyAsyncShared();
       };
-      if (i >= (kSplitP ? 1 : 2)) ok = WarpSpin(bar(&misc->s_empty[buf]), ((kSplitP ? i : i >> 1) & 1) ^ 1, misc, p.status, 228);
+      if (i >= (kSplitP ? 1 : 2)) ok = WarpWait(bar(&misc->s_empty[buf]), ((kSplitP ? i : i >> 1) & 1) ^ 1, misc, p.status, 228);
       if (ok) group_ready(0);
       if (!ok) break;
       IssueQkGroup<0, 2, kSplitP>(q_desc, kdesc, d);
@@ -546,7 +539,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       if (valid < kTile) {
         // Rows past the sequence's end hold whatever the pool held; zero them so 0 * NaN cannot reach O. This warp has
         // nothing else to do until P is there. (QK may still be reading these rows; their scores are masked.)
-        for (int c = 0; c < kGroups && ok; ++c) ok = WarpSpin(bar(&misc->kv_full[stage][c]), (i / kStages) & 1, misc, p.status, 220);
+        for (int c = 0; c < kGroups && ok; ++c) ok = WarpWait(bar(&misc->kv_full[stage][c]), (i / kStages) & 1, misc, p.status, 220);
         if (!ok) break;
         unsigned char* stage_ptr = smem + kOffKv + stage * kStageBytes;
         for (int idx = lane; idx < (kTile - valid) * 64; idx += 32) {
@@ -555,7 +548,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         ptx::FenceProxyAsyncShared();
         __syncwarp();
       }
-      ok = WarpSpin(bar(&misc->p_full[stage]), (i / kStages) & 1, misc, p.status, 221);
+      ok = WarpWait(bar(&misc->p_full[stage]), (i / kStages) & 1, misc, p.status, 221);
       if (!ok) break;
       ptx::TcFenceAfterSync();
       if constexpr (kCopied) ptx::FenceProxyAsyncShared();
@@ -587,7 +580,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     for (int i = 0; i < n; ++i) {
       const int buf = kSplitP ? 0 : i & 1, stage = i % kStages;
       const int valid = min(kTile, len - (share.t_lo + i) * kTile);
-      ok = WarpSpin(bar(&misc->s_full[buf]), (kSplitP ? i : i >> 1) & 1, misc, p.status, 230);
+      ok = WarpWait(bar(&misc->s_full[buf]), (kSplitP ? i : i >> 1) & 1, misc, p.status, 230);
       if (!ok) break;
       ptx::TcFenceAfterSync();
       uint32_t sr[32];
@@ -673,7 +666,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       if (i > 0 && (any_rescale || kSplitP)) {
         // PV of the previous tile must have drained: before its accumulators are rescaled (rare), and before the one
         // buffer of P's low term is written again. (It ran under this tile's exponentials.)
-        ok = WarpSpin(bar(&misc->kv_empty[(i - 1) % kStages][kGroups - 1]), ((i - 1) / kStages) & 1, misc, p.status, 231);
+        ok = WarpWait(bar(&misc->kv_empty[(i - 1) % kStages][kGroups - 1]), ((i - 1) / kStages) & 1, misc, p.status, 231);
         if (!ok) break;
         ptx::TcFenceAfterSync();
       }
@@ -713,7 +706,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       __syncwarp();
       if (lane == 0) ptx::MbarArrive(bar(&misc->p_full[stage]));
     }
-    if (ok) ok = WarpSpin(bar(&misc->o_full), 0, misc, p.status, 232);
+    if (ok) ok = WarpWait(bar(&misc->o_full), 0, misc, p.status, 232);
     ptx::TcFenceAfterSync();
   }
   if (warp == 5 || warp == 6) {
@@ -737,6 +730,9 @@ __global__ void __launch_bounds__(kThreads, 1)
   const int quads = share.heads >> 2;
   const int first = head_first + share.head_lo;
   const bool want_partial = p.user_o != nullptr;
+  // What every call of an engine is: bf16 rows of whole heads, nothing else. The code for it is kept to the instructions
+  // that do the work (a warp alone on its scheduler takes some six cycles for each); the rest goes through `emit`.
+  const bool plain = !want_partial && p.out_q == nullptr && first + share.heads <= p.heads;
   // Four heads of one output column: lane = column, so an output store of the warp is 64 contiguous bytes of a row.
   auto emit = [&](int quad, int dv, const float (&acc)[4]) {  // every lane of the warp calls
     const int64_t row0 = static_cast<int64_t>(seq) * p.heads + first + 4 * quad;
@@ -794,14 +790,14 @@ __global__ void __launch_bounds__(kThreads, 1)
   // The accumulators: warp w reads lanes 32 (w % 4) .. of numbers w / 4 and w / 4 + 2.
   const uint32_t acc_base = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16) + 64 * (warp >> 2);
   const int dv_warp = 128 * (warp >> 2) + 32 * (warp & 3);  // output column of lane 0 in the first of the two, + 256 in the other
-  if (n > 0 && warp >= 4) WarpSpin(bar(&misc->o_full), 0, misc, p.status, 233);
+  if (n > 0 && warp >= 4) WarpWait(bar(&misc->o_full), 0, misc, p.status, 233);
   ptx::ClusterWait();
 
-  if (share.ranges == 1) {
+  if (share.ranges == 1 && plain) {
     // Nobody to exchange with: out of the accumulators straight into the rows.
     float* s_norm = reinterpret_cast<float*>(smem + kOffW);
     if (has_row) {
-      s_norm[h_row] = want_partial ? 1.0f : (l_row > 0.0f ? 1.0f / l_row : 0.0f);
+      s_norm[h_row] = l_row > 0.0f ? 1.0f / l_row : 0.0f;
       emit_ml(h_row, m_row, l_row);
     }
     __syncthreads();
@@ -813,17 +809,20 @@ __global__ void __launch_bounds__(kThreads, 1)
       uint32_t o[32];
       ptx::TmemLd32(acc_base + 128 * (part >> 1) + 32 * half, o);
       ptx::TmemWaitLd();
+      if (n == 0) {
+#pragma unroll
+        for (int q = 0; q < 32; ++q) o[q] = 0u;  // an empty sequence: nothing was accumulated
+      }
+      __nv_bfloat16* dst = p.out + (static_cast<int64_t>(seq) * p.heads + first + 32 * half) * kLatent + dv;
+      const float4* norm = reinterpret_cast<const float4*>(s_norm + 32 * half);
 #pragma unroll
       for (int q = 0; q < 8; ++q) {
-        const int quad = 8 * half + q;
-        if (quad >= quads || first + 4 * quad >= p.heads) break;
-        const float4 w = *reinterpret_cast<const float4*>(&s_norm[4 * quad]);
-        float acc[4];
-        acc[0] = n > 0 ? __uint_as_float(o[4 * q]) * w.x : 0.0f;
-        acc[1] = n > 0 ? __uint_as_float(o[4 * q + 1]) * w.y : 0.0f;
-        acc[2] = n > 0 ? __uint_as_float(o[4 * q + 2]) * w.z : 0.0f;
-        acc[3] = n > 0 ? __uint_as_float(o[4 * q + 3]) * w.w : 0.0f;
-        emit(quad, dv, acc);
+        if (q == 4 && share.heads == kLeastHeads) break;
+        const float4 w = norm[q];
+        dst[(4 * q) * kLatent] = __float2bfloat16_rn(__uint_as_float(o[4 * q]) * w.x);
+        dst[(4 * q + 1) * kLatent] = __float2bfloat16_rn(__uint_as_float(o[4 * q + 1]) * w.y);
+        dst[(4 * q + 2) * kLatent] = __float2bfloat16_rn(__uint_as_float(o[4 * q + 2]) * w.z);
+        dst[(4 * q + 3) * kLatent] = __float2bfloat16_rn(__uint_as_float(o[4 * q + 3]) * w.w);
       }
     }
     ptx::TcFenceBeforeSync();
@@ -905,17 +904,19 @@ __global__ void __launch_bounds__(kThreads, 1)
   float4* s_w = reinterpret_cast<float4*>(smem + kOffW) + warp * kMaxCluster;  // [range] of the warp's present quad
   const int groups_log2 = columns_log2 - 5;  // columns / 32
   const int units = quads << groups_log2;
-  const int unit_lo = units * warp / kWarps, unit_hi = units * (warp + 1) / kWarps;
+  const int unit_hi = units * (warp + 1) / kWarps;
   const float4* mail = reinterpret_cast<const float4*>(smem + mail_off);
   int have_quad = -1;
-  for (int unit = unit_lo; unit < unit_hi; ++unit) {
-    const int quad = unit >> groups_log2, local = ((unit & ((1 << groups_log2) - 1)) << 5) + lane;
+  bool whole = false;  // every range has a weight for each of the quad's heads
+  for (int unit = units * warp / kWarps; unit < unit_hi; ++unit) {
+    const int quad = unit >> groups_log2, group = unit & ((1 << groups_log2) - 1);
     if (first + 4 * quad >= p.heads) break;  // (units walk the quads upwards)
     if (quad != have_quad) {
       have_quad = quad;
       const int h = 4 * quad + (lane & 3);
       float m[2], l[2];
       float big = -INFINITY, total = 0.0f;
+      bool zero = false;
 #pragma unroll
       for (int k = 0; k < 2; ++k) {
         const int s = (lane >> 2) + 8 * k;
@@ -928,32 +929,53 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
       for (int k = 0; k < 2; ++k) {
         m[k] = l[k] > 0.0f ? exp2f(m[k] - big) : 0.0f;  // the range's weight
+        zero |= (lane >> 2) + 8 * k < share.ranges && !(m[k] > 0.0f);
         total = fmaf(l[k], m[k], total);
       }
 #pragma unroll
       for (int off = 4; off < 32; off <<= 1) total += __shfl_xor_sync(0xffffffffu, total, off);
-      __syncwarp();  // the previous quad's weights have been read
+      whole = !__any_sync(0xffffffffu, zero);  // (and: the previous quad's weights have been read)
       const float norm = want_partial ? 1.0f : (total > 0.0f ? 1.0f / total : 0.0f);
 #pragma unroll
       for (int k = 0; k < 2; ++k) {
         const int s = (lane >> 2) + 8 * k;
         if (s < share.ranges) reinterpret_cast<float*>(s_w)[4 * s + (lane & 3)] = m[k] * norm;
       }
-      if (share.range == 0 && lane < 4 && (unit & ((1 << groups_log2) - 1)) == 0) emit_ml(h, big, total);
+      if (share.range == 0 && lane < 4 && group == 0) emit_ml(h, big, total);
       __syncwarp();
     }
+    const int local = group * kDvGroup + lane;
+    const float4* row = &mail[(quad << columns_log2) + local];
+    const int step = quads << columns_log2;  // from one range to the next
     float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    if (whole) {
 #pragma unroll 4
-    for (int s = 0; s < share.ranges; ++s) {
-      const float4 w = s_w[s];
-      const float4 v = mail[((s * quads + quad) << columns_log2) + local];
-      // A range without tiles sent nothing: its weight is zero and its place holds anything.
-      acc[0] = fmaf(w.x != 0.0f ? v.x : 0.0f, w.x, acc[0]);
-      acc[1] = fmaf(w.y != 0.0f ? v.y : 0.0f, w.y, acc[1]);
-      acc[2] = fmaf(w.z != 0.0f ? v.z : 0.0f, w.z, acc[2]);
-      acc[3] = fmaf(w.w != 0.0f ? v.w : 0.0f, w.w, acc[3]);
+      for (int s = 0; s < share.ranges; ++s) {
+        const float4 w = s_w[s], v = row[s * step];
+        acc[0] = fmaf(v.x, w.x, acc[0]);
+        acc[1] = fmaf(v.y, w.y, acc[1]);
+        acc[2] = fmaf(v.z, w.z, acc[2]);
+        acc[3] = fmaf(v.w, w.w, acc[3]);
+      }
+    } else {
+#pragma unroll 1
+      for (int s = 0; s < share.ranges; ++s) {
+        const float4 w = s_w[s], v = row[s * step];
+        // A range without tiles sent nothing: its weight is zero and its place holds anything.
+        acc[0] = fmaf(w.x != 0.0f ? v.x : 0.0f, w.x, acc[0]);
+        acc[1] = fmaf(w.y != 0.0f ? v.y : 0.0f, w.y, acc[1]);
+        acc[2] = fmaf(w.z != 0.0f ? v.z : 0.0f, w.z, acc[2]);
+        acc[3] = fmaf(w.w != 0.0f ? v.w : 0.0f, w.w, acc[3]);
+      }
     }
-    emit(quad, (share.range << columns_log2) + local, acc);
+    const int dv = (share.range << columns_log2) + local;
+    if (plain) {
+      __nv_bfloat16* dst = p.out + (static_cast<int64_t>(seq) * p.heads + first + 4 * quad) * kLatent + dv;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) dst[i * kLatent] = __float2bfloat16_rn(acc[i]);
+    } else {
+      emit(quad, dv, acc);
+    }
   }
 }
 
