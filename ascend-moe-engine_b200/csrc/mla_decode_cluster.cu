@@ -1116,17 +1116,16 @@ int32_t Launch(const b200kv_decode_args& a, int source, bool split_p, int32_t cl
 
 // Up to how many tiles in its longest sequence a batch is better off here than in the flat kernel, which spreads all
 // tiles over all SMs but pays for two launches and the merge of every sequence's parts. Both sides measured (us a layer,
-// flat -> here, all sequences of the length / lengths from a sixteenth of it):
-//   16 CTAs  1 x 2,048: 16.3 -> 16.4, 1 x 4,096: 16.5 -> 19.9; 2 x 4,096: 22.1 -> 20.3, 4 x 4,096: 25.2 -> 20.9 / 24.4 -> 18.9
-//            (three or four sequences of many parts are the merge kernel's worst case); 8 x 2,048: 21.3 -> 19.9, 8 x 4,096:
-//            25.1 -> 27.3
-//    8 CTAs  16 x 1,024: 21.4 -> 19.5 / 20.6 -> 19.2, 16 x 2,048: 25.1 -> 26.7
-//    4 CTAs  32 x 1,024: 23.2 -> 21.8 / 21.1 -> 20.7, 32 x 4,096: 45.2 -> 44.9 / 33.8 -> 42.6
-//    2 CTAs  64 x 512: 27.9 -> 22.5 / 24.2 -> 22.0, 64 x 1,024: 34.8 -> 30.5
-//    1 CTA   128 x 512: 42.1 -> 29.2; 140 x 512: / 38.2 -> 31.5; 128 x 1,024: 56.9 -> 44.8
+// flat -> here; all sequences of the length / lengths from a sixteenth of it):
+//   16 CTAs  1 x 2,048: 15.7 -> 15.9, 1 x 4,096: 16.1 -> 19.5; 2 x 2,048: 20.5 -> 15.9, 2 x 4,096: 21.5 -> 19.8; 3 x 4,096:
+//            17.5 -> 19.8; 4 x 2,048: 18.5 -> 16.4
+//    8 CTAs  12 x 1,024: 17.5 -> 16.4; 8 x 2,048: 18.9 -> 19.2
+//    4 CTAs  16 x 1,024: 18.5 -> 18.6, 32 x 1,024: 22.5 -> 21.1 / 20.3 -> 20.1; 32 x 4,096: 44.3 -> 43.9 / 33.1 -> 42.6
+//    2 CTAs  64 x 512: 27.4 -> 21.7 / 23.9 -> 21.0, 64 x 768: / 26.7 -> 25.6
+//    1 CTA   128 x 512: 41.5 -> 25.7; in more than one wave 256 x 512: 65.9 -> 56.6, 600 x 64: 68.8 -> 60.9
 int64_t MostTilesFor(int32_t cluster, int32_t batch) {
   switch (cluster) {
-    case 16: return batch >= 2 && batch <= 4 ? 64 : 32;
+    case 16: return batch == 2 ? 64 : 32;
     case 8: return 16;
     case 4: return 16;
     case 2: return 12;

@@ -126,6 +126,14 @@ struct TcParams {
   int32_t* status;
 };
 
+// A bounded wait by all lanes of a warp together, behind an inline probe: a phase that is complete already (the usual case
+// for a tile's later slab groups) costs no call. 45.2 -> 44.2 us for 32 sequences of 4,096 tokens, 17.4 -> 16.9 us for one
+// of 8,192.
+__device__ __forceinline__ bool WarpWait(uint32_t bar, uint32_t parity, Misc* misc, int32_t* status, int site) {
+  if (__all_sync(0xffffffffu, ptx::MbarTestWait(bar, parity))) return true;
+  return __all_sync(0xffffffffu, BoundedWait(bar, parity, misc, status, site));
+}
+
 // ---- work partition -----------------------------------------------------------------------------------
 // The tiles of all sequences form one flat list (sequence after sequence, empty ones contribute nothing).
 // Cutting that list into G equal runs of tiles leaves the CTAs uneven: a CTA whose run crosses from one
@@ -537,7 +545,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         // Q of this segment's sequence, once the previous segment's last QK has finished reading the
         // buffer (the first segment's Q went out before the setup barrier).
         if (seg > 0) {
-          ok = __all_sync(0xffffffffu, BoundedWait(bar(&misc->q_empty), (seg - 1) & 1, misc, p.status, 11));
+          ok = WarpWait(bar(&misc->q_empty), (seg - 1) & 1, misc, p.status, 11);
           if (!ok) break;
           if (loader) issue_q(seq);
         }
@@ -682,7 +690,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             const int stage = g % kStages;
             const int buf = g & 1;
             const uint32_t kv_parity = (g / kStages) & 1;
-            ok = __all_sync(0xffffffffu, BoundedWait(bar(&misc->kv_full[stage][0]), kv_parity, misc, p.status, 24));
+            ok = WarpWait(bar(&misc->kv_full[stage][0]), kv_parity, misc, p.status, 24);
             if (ok && g >= 2) {
               ok = __all_sync(0xffffffffu,
                               BoundedWait(bar(&misc->s_empty[buf]), ((g >> 1) & 1) ^ 1, misc, p.status, 25));
@@ -690,7 +698,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             // A segment's first tile also waits, group by group, for the sequence's Q.
             const bool first_of_segment = i == 0;
             if (ok && first_of_segment) {
-              ok = __all_sync(0xffffffffu, BoundedWait(bar(&misc->q_full[0]), seg & 1, misc, p.status, 22));
+              ok = WarpWait(bar(&misc->q_full[0]), seg & 1, misc, p.status, 22);
             }
             if (!ok) break;
             ptx::TcFenceAfterSync();
@@ -700,25 +708,25 @@ __global__ void __launch_bounds__(kThreads, 1)
             // Twelve k-steps per slab group, each group as soon as its slabs have landed (compile-time
             // offsets; a runtime offset costs the uniform-datapath issue rate).
             IssueQkGroup<0, 2>(q_desc, kdesc, d);
-            ok = __all_sync(0xffffffffu, BoundedWait(bar(&misc->kv_full[stage][1]), kv_parity, misc, p.status, 26));
+            ok = WarpWait(bar(&misc->kv_full[stage][1]), kv_parity, misc, p.status, 26);
             if (ok && first_of_segment) {
-              ok = __all_sync(0xffffffffu, BoundedWait(bar(&misc->q_full[1]), seg & 1, misc, p.status, 22));
+              ok = WarpWait(bar(&misc->q_full[1]), seg & 1, misc, p.status, 22);
             }
             if (!ok) break;
             ptx::TcFenceAfterSync();
             if constexpr (kGathered) ptx::FenceProxyAsyncShared();
             IssueQkGroup<2, 2>(q_desc, kdesc, d);
-            ok = __all_sync(0xffffffffu, BoundedWait(bar(&misc->kv_full[stage][2]), kv_parity, misc, p.status, 27));
+            ok = WarpWait(bar(&misc->kv_full[stage][2]), kv_parity, misc, p.status, 27);
             if (ok && first_of_segment) {
-              ok = __all_sync(0xffffffffu, BoundedWait(bar(&misc->q_full[2]), seg & 1, misc, p.status, 22));
+              ok = WarpWait(bar(&misc->q_full[2]), seg & 1, misc, p.status, 22);
             }
             if (!ok) break;
             ptx::TcFenceAfterSync();
             if constexpr (kGathered) ptx::FenceProxyAsyncShared();
             IssueQkGroup<4, 2>(q_desc, kdesc, d);
-            ok = __all_sync(0xffffffffu, BoundedWait(bar(&misc->kv_full[stage][3]), kv_parity, misc, p.status, 28));
+            ok = WarpWait(bar(&misc->kv_full[stage][3]), kv_parity, misc, p.status, 28);
             if (ok && first_of_segment) {
-              ok = __all_sync(0xffffffffu, BoundedWait(bar(&misc->q_full[3]), seg & 1, misc, p.status, 22));
+              ok = WarpWait(bar(&misc->q_full[3]), seg & 1, misc, p.status, 22);
             }
             if (!ok) break;
             ptx::TcFenceAfterSync();
@@ -732,7 +740,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         } else {
           if (seg > 0) {
             // The previous segment's accumulators must have been drained by the epilogue.
-            ok = __all_sync(0xffffffffu, BoundedWait(bar(&misc->o_empty), (seg - 1) & 1, misc, p.status, 23));
+            ok = WarpWait(bar(&misc->o_empty), (seg - 1) & 1, misc, p.status, 23);
           }
           for (int i = 0; i < n && ok; ++i) {
             const int g = __shfl_sync(0xffffffffu, g0 + i, 0);
@@ -1027,10 +1035,11 @@ __global__ void __launch_bounds__(kThreads, 1)
 // loads of the chunk's first parts are issued, one warp per part group works out the weights of its eight parts
 // for the quad's four heads (lane = part x head; the maxima and sums are shuffles) and leaves them in shared
 // memory, and every thread accumulates weight x data.
-// kGroups = 1: 128 threads, 256 columns per CTA in two passes, every thread walks all parts (batches, where a
-// sequence has a handful of parts: 32 CTAs per sequence). kGroups = 8: 256 threads, 32 columns per CTA, a
-// chunk is 256 parts of which each warp takes 32 consecutive ones, summed through shared memory at the end
-// (a few long sequences with a hundred parts each: 256 CTAs per sequence, one chunk, one round of weights).
+// kGroups: how many groups of a CTA's threads share a sequence's parts out (part i goes to group i % kGroups, summed through
+// shared memory at the end), kPasses: columns per thread. Both follow from the batch, which says how many parts a
+// sequence has (about 148 / batch + 1) and how many columns there are to work on: the shape is chosen so that some 130
+// thousand threads, what the register files hold, have all parts but a few in flight at once. kResident: CTAs an SM
+// is to hold. kRuns: a group takes 32 consecutive parts instead (one sequence's 148: 0.5 us shorter).
 // The kernel needs a few hundred bytes of shared memory, so its CTAs fit beside a resident decode CTA.
 //
 // kPeer (with kGroups = 8): the sequence is a KV-range shard of a longer one that other GPUs hold the rest of.
@@ -1038,18 +1047,17 @@ __global__ void __launch_bounds__(kThreads, 1)
 // over peer memory, and the same threads then wait (bounded) for the other ranks' words of their columns,
 // merge them and write the final rows: the exchange protocol of kv_peer.cu without a kernel, and a pass over
 // the partial, in between. A thread waits only for words that other GPUs' kernels write.
-template <int kGroups, bool kPeer = false, bool kQuant = false>
-__global__ void __launch_bounds__(kGroups == 1 ? 128 : 256, kGroups == 1 ? 7 : 2)
+template <int kGroups, int kPasses, int kResident, bool kRuns, bool kPeer, bool kQuant>
+__global__ void __launch_bounds__(kGroups == 1 ? 128 : 256, kResident)
     MlaFinalizeKernel(TcParams p, int32_t n_ctas, PeerRing ring) {
   static_assert(!kPeer || kGroups == 8, "the peer form is built on the few-sequences variant");
   constexpr int kThreadsF = kGroups == 1 ? 128 : 256;
-  constexpr int kGroupThreads = kThreadsF / kGroups;   // 128 or 32: columns a group covers per pass
-  constexpr int kPasses = kGroups == 1 ? 2 : 1;
-  constexpr int kDv = kGroupThreads * kPasses;         // 256 or 32 output columns per CTA
-  constexpr int kGroupParts = kGroups == 1 ? 8 : 32;   // parts of a chunk that one group takes
-  constexpr int kChunk = kGroupParts * kGroups;        // parts per chunk: 8, or 256 (a long sequence's in one go)
+  constexpr int kGroupThreads = kThreadsF / kGroups;   // columns a group covers per pass
+  constexpr int kDv = kGroupThreads * kPasses;         // output columns per CTA: 256, 128, 64 or 32
+  constexpr int kGroupParts = kPasses == 2 ? 8 : (kGroups == 8 ? 32 : 16);  // parts of a chunk that one group takes
+  constexpr int kChunk = kGroupParts * kGroups;        // parts per chunk
   constexpr int kRounds = kGroupParts / 8;             // a warp works out the weights of 8 parts x 4 heads at a time
-  constexpr int kSub = kGroups == 1 ? 4 : 8;           // parts whose data a thread has in flight
+  constexpr int kSub = kPasses == 2 ? 4 : 8;           // parts whose data a thread has in flight
   constexpr int kDvChunks = kLatent / kDv;             // 2 or 16
   constexpr int kQuads = kHeads / 4;
 
@@ -1136,6 +1144,8 @@ __global__ void __launch_bounds__(kGroups == 1 ? 128 : 256, kGroups == 1 ? 7 : 2
   // one tile (consecutive tiles are at most 5 units apart), so every CTA from the first to the last holds a
   // part and no division is needed.
   const bool dense = cut.cost_total >= (CostCut::kTileCost + CostCut::kCrossCost) * cut.n_ctas;
+  // Place in the chunk of a group's i-th part.
+  auto part_at = [](int group_, int i) { return kRuns ? group_ * kGroupParts + i : i * kGroups + group_; };
   auto slot_of = [&](int c) {
     if (c > cl) return -1;
     if (!dense) {
@@ -1177,12 +1187,12 @@ __global__ void __launch_bounds__(kGroups == 1 ? 128 : 256, kGroups == 1 ? 7 : 2
     if (c0 != cf) __syncthreads();  // the previous chunk's weights and slots have been used
     if (tid < kChunk) s_slot[tid] = slot_of(c0 + tid);
     __syncthreads();
-    // This thread's parts of the chunk: kGroupParts consecutive ones per group, kSub at a time.
+      // This thread's parts of the chunk, kSub at a time.
     float4 data[kSub][kPasses];
     auto load_sub = [&](int sub) {
 #pragma unroll
       for (int k = 0; k < kSub; ++k) {
-        const int slot = s_slot[group * kGroupParts + sub * kSub + k];
+        const int slot = s_slot[part_at(group, sub * kSub + k)];
 #pragma unroll
         for (int q = 0; q < kPasses; ++q) {
           data[k][q] = slot >= 0 ? ws4[(static_cast<int64_t>(slot) * kQuads + hq) * kLatent + dv_first + kGroupThreads * q]
@@ -1198,7 +1208,7 @@ __global__ void __launch_bounds__(kGroups == 1 ? 128 : 256, kGroups == 1 ? 7 : 2
       float gmax = -INFINITY;
 #pragma unroll
       for (int r = 0; r < kRounds; ++r) {
-        const int slot = s_slot[warp * kGroupParts + 8 * r + (lane >> 2)];
+        const int slot = s_slot[part_at(warp, 8 * r + (lane >> 2))];
         m_mine[r] = -INFINITY;
         l_mine[r] = 0.0f;
         if (slot >= 0) {
@@ -1226,7 +1236,7 @@ __global__ void __launch_bounds__(kGroups == 1 ? 128 : 256, kGroups == 1 ? 7 : 2
 #pragma unroll
       for (int r = 0; r < kRounds; ++r) {
         const float w = (l_mine[r] > 0.0f && new_big != -INFINITY) ? expf(m_mine[r] - new_big) : 0.0f;
-        s_w[warp * kGroupParts + 8 * r + (lane >> 2)][i] = w;
+        s_w[part_at(warp, 8 * r + (lane >> 2))][i] = w;
         gsum = fmaf(l_mine[r], w, gsum);
       }
 #pragma unroll
@@ -1264,14 +1274,14 @@ __global__ void __launch_bounds__(kGroups == 1 ? 128 : 256, kGroups == 1 ? 7 : 2
 #pragma unroll 1
     for (int sub = 0; sub < kGroupParts / kSub; ++sub) {
       if (sub > 0) {
-        if (s_slot[group * kGroupParts + sub * kSub] < 0 && dense) break;  // dense: parts are consecutive, the rest is absent
+        if (s_slot[part_at(group, sub * kSub)] < 0 && dense) break;  // dense: parts are consecutive, the rest is absent
         load_sub(sub);
       }
 #pragma unroll
       for (int k = 0; k < kSub; ++k) {
         // An absent part has weight zero and zero data; a present one with l = 0 may hold anything (0 x NaN is
         // not 0), so its data is dropped with its weight.
-        const float4 w = *reinterpret_cast<const float4*>(s_w[group * kGroupParts + sub * kSub + k]);
+        const float4 w = *reinterpret_cast<const float4*>(s_w[part_at(group, sub * kSub + k)]);
 #pragma unroll
         for (int q = 0; q < kPasses; ++q) {
           acc[q][0] = fmaf(w.x != 0.0f ? data[k][q].x : 0.0f, w.x, acc[q][0]);
@@ -1724,27 +1734,38 @@ int32_t LaunchMlaDecodeTc(const b200kv_decode_args& a, int32_t n_ctas, cudaStrea
                              "tcgen05 decode launch")) {
     return rc;
   }
-  // One or two long sequences: 256 CTAs per sequence, the parts shared out among a CTA's eight warps, so that
-  // the merge still fills the GPU. Batches: 32 CTAs per sequence, every thread walking the sequence's parts.
+  // The merge's shape by the number of sequences (see the kernel): groups x passes, chosen so that one wave of CTAs
+  // holds the launch (three or four of 256 threads on an SM) and a thread has few parts to walk. us a layer with the form
+  // for one or two sequences up to two, one group and two passes above, and now: 2 x 16,384 tokens 27.1 -> 26.1, 3 x 16,384
+  // 35.3 -> 27.0, 5 x 8,192 29.7 -> 24.9, 8 x 8,192 31.0 -> 30.4, 12 x 4,096 29.5 -> 27.0, 16 x 4,096 31.9 -> 30.6. (Eight
+  // sequences with three CTAs of two groups on an SM: 32.0, a second wave; one group and one pass from 17 sequences on the
+  // same. The exchange across GPUs exists in the form for one sequence only.)
   const bool quant = p.out_q != nullptr;
-  const dim3 grid_few(static_cast<unsigned>(a.batch) * 16 * (kLatent / 32)), grid_many(static_cast<unsigned>(a.batch) * 16 * (kLatent / 256));
   cudaError_t launched;
   const char* what = "decode finalize launch";
-  // (The 256-CTA form runs two CTAs per SM: one sequence is one wave, two are two, and from three on the
-  // 32-CTA form, whose threads walk a sequence's parts eight at a time, is the shorter one. The exchange across
-  // GPUs exists in the 256-CTA form only.)
-  if (a.batch < 3 || ring != nullptr) {
-    if (ring != nullptr) {
-      what = "decode finalize + peer merge launch";
-      launched = quant ? LaunchOverlapped(MlaFinalizeKernel<8, true, true>, grid_few, dim3(256), 0, stream, p, n_ctas, *ring)
-                       : LaunchOverlapped(MlaFinalizeKernel<8, true, false>, grid_few, dim3(256), 0, stream, p, n_ctas, *ring);
-    } else {
-      launched = quant ? LaunchOverlapped(MlaFinalizeKernel<8, false, true>, grid_few, dim3(256), 0, stream, p, n_ctas, PeerRing{})
-                       : LaunchOverlapped(MlaFinalizeKernel<8, false, false>, grid_few, dim3(256), 0, stream, p, n_ctas, PeerRing{});
-    }
+  auto launch = [&](auto kernel, auto quant_kernel, int columns, int threads, const PeerRing& r) {
+    const dim3 grid(static_cast<unsigned>(a.batch) * 16 * static_cast<unsigned>(kLatent / columns));
+    return quant ? LaunchOverlapped(quant_kernel, grid, dim3(threads), 0, stream, p, n_ctas, r)
+                 : LaunchOverlapped(kernel, grid, dim3(threads), 0, stream, p, n_ctas, r);
+  };
+  const PeerRing none{};
+  if (ring != nullptr) {
+    what = "decode finalize + peer merge launch";
+    launched = launch(MlaFinalizeKernel<8, 1, 2, true, true, false>, MlaFinalizeKernel<8, 1, 2, true, true, true>, 32, 256, *ring);
+  } else if (a.batch == 1) {
+    launched = launch(MlaFinalizeKernel<8, 1, 2, true, false, false>, MlaFinalizeKernel<8, 1, 2, true, false, true>, 32, 256, none);
+  } else if (a.batch == 2) {
+    launched = launch(MlaFinalizeKernel<8, 1, 2, false, false, false>, MlaFinalizeKernel<8, 1, 2, false, false, true>, 32, 256, none);
+  } else if (a.batch == 3) {
+    launched = launch(MlaFinalizeKernel<4, 1, 3, false, false, false>, MlaFinalizeKernel<4, 1, 3, false, false, true>, 64, 256, none);
+  } else if (a.batch <= 6) {
+    launched = launch(MlaFinalizeKernel<2, 1, 3, false, false, false>, MlaFinalizeKernel<2, 1, 3, false, false, true>, 128, 256, none);
+  } else if (a.batch <= 8) {
+    launched = launch(MlaFinalizeKernel<2, 1, 4, false, false, false>, MlaFinalizeKernel<2, 1, 4, false, false, true>, 128, 256, none);
+  } else if (a.batch <= 16) {
+    launched = launch(MlaFinalizeKernel<1, 1, 7, false, false, false>, MlaFinalizeKernel<1, 1, 7, false, false, true>, 128, 128, none);
   } else {
-    launched = quant ? LaunchOverlapped(MlaFinalizeKernel<1, false, true>, grid_many, dim3(128), 0, stream, p, n_ctas, PeerRing{})
-                     : LaunchOverlapped(MlaFinalizeKernel<1, false, false>, grid_many, dim3(128), 0, stream, p, n_ctas, PeerRing{});
+    launched = launch(MlaFinalizeKernel<1, 2, 7, false, false, false>, MlaFinalizeKernel<1, 2, 7, false, false, true>, 256, 128, none);
   }
   return CheckCuda(launched, what);
 }

@@ -123,3 +123,37 @@ def test_any_geometry_reports_a_length_beyond_the_table():
     torch.cuda.synchronize()
     got = status.cpu().tolist()
     assert got[0] == b200kv.DEV_BAD_BLOCK and got[1] == 1, got
+
+
+@pytest.mark.parametrize("batch", [1, 2, 3, 4, 6, 7, 8, 9, 16, 17])
+@pytest.mark.parametrize("quantised", [False, True])
+def test_merge_of_many_parts_in_every_shape(batch, quantised):
+    """Histories beyond the cluster form's: partials of every CTA, merged in the shape that the batch selects. Against the
+    CUDA-core kernel (fp32 weights, its own merge): bf16 results of the same rows, whose weights the tensor-core kernel
+    rounds to bf16 (2^-9 of values of magnitude 4 at most)."""
+    bs = 64
+    kv_len = np.array([9000 - 517 * (i % 9) if i != 1 else 65 for i in range(batch)], dtype=np.int32)
+    blocks = int(sum(scenarios.blocks_for(int(n), bs) for n in kv_len)) + 3
+    table = scenarios.build_tables(kv_len, bs, blocks, order=kvo.permutation(blocks))
+    g = torch.Generator(device="cuda")
+    g.manual_seed(batch)
+    pool = torch.randn((blocks * bs, 576), generator=g, device="cuda").bfloat16()
+    q = torch.randn((batch, 64, 576), generator=g, device="cuda").bfloat16()
+    d_table, d_len = to_dev_i32(table), to_dev_i32(kv_len)
+    ws = torch.empty(b200kv.decode_workspace_bytes(batch), dtype=torch.uint8, device="cuda")
+    status = b200kv.new_status()
+    got = []
+    for variant in (b200kv.DECODE_TCGEN05, b200kv.DECODE_SIMT):
+        out = torch.full((batch, 64, 512), float("nan"), dtype=torch.bfloat16, device="cuda")
+        lse = torch.full((batch, 64), float("nan"), dtype=torch.float32, device="cuda")
+        codes = (torch.zeros((batch, 64, 512), dtype=torch.uint8, device="cuda"), torch.zeros((batch, 64, 16), dtype=torch.uint8, device="cuda"))
+        b200kv.mla_decode(q, b200kv.pool_view(pool), d_table, d_len, bs, 1.0 / 24.0, out=out, lse=lse, workspace=ws, status=status,
+                          variant=variant, quantised=codes if quantised else None)
+        status_ok(status)
+        got.append((out.float(), lse))
+        if quantised:
+            fp8, scales = torch.empty((batch, 64 * 512), dtype=torch.uint8, device="cuda"), torch.empty((batch, 1024), dtype=torch.uint8, device="cuda")
+            b200kv.mx_quant_e4m3(out.view(batch, -1), fp8, scales)
+            assert torch.equal(codes[0].view(batch, -1), fp8) and torch.equal(codes[1].view(batch, -1), scales)
+    assert ((got[0][0] - got[1][0]).abs() <= 2e-3 + 1e-2 * got[1][0].abs().amax(dim=2, keepdim=True)).all()
+    assert ((got[0][1] - got[1][1]).abs() <= 1e-4).all()
