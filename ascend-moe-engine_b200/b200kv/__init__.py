@@ -8,6 +8,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+import struct
 from ctypes import POINTER, Structure, c_char_p, c_double, c_float, c_int32, c_int64, c_size_t, c_uint64, c_void_p
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
@@ -142,16 +143,16 @@ def _load() -> ctypes.CDLL:
     lib.b200kv_mla_decode_workspace_bytes.restype = c_size_t
     lib.b200kv_mla_decode_workspace_bytes.argtypes = [c_int32, c_int32, c_int32]
     lib.b200kv_mla_decode.restype = c_int32
-    lib.b200kv_mla_decode.argtypes = [POINTER(DecodeArgs), c_void_p, c_void_p]
+    lib.b200kv_mla_decode.argtypes = [c_void_p, c_void_p, c_void_p]
     lib.b200kv_append_fused.restype = c_int32
-    lib.b200kv_append_fused.argtypes = [POINTER(ProducerArgs), c_void_p, c_void_p]
+    lib.b200kv_append_fused.argtypes = [c_void_p, c_void_p, c_void_p]
     lib.b200kv_mx_quant_e4m3.restype = c_int32
     lib.b200kv_mx_quant_e4m3.argtypes = [c_void_p, c_int64, c_int64, c_int64, c_void_p, c_int64, c_void_p, c_int64,
                                          c_void_p]
     lib.b200kv_indexer_workspace_bytes.restype = c_size_t
     lib.b200kv_indexer_workspace_bytes.argtypes = [c_int32, c_int64]
     lib.b200kv_indexer_topk.restype = c_int32
-    lib.b200kv_indexer_topk.argtypes = [POINTER(IndexerArgs), c_void_p, c_void_p]
+    lib.b200kv_indexer_topk.argtypes = [c_void_p, c_void_p, c_void_p]
     lib.b200kv_resolve_rows.restype = c_int32
     lib.b200kv_resolve_rows.argtypes = [c_void_p, c_int64, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_int64,
                                         c_void_p, c_void_p, c_void_p]
@@ -215,15 +216,32 @@ def check(code: int) -> None:
 # ---------------------------------------------------------------------------------------------------
 # Device operations on torch tensors
 # ---------------------------------------------------------------------------------------------------
-def _stream_handle(stream=None) -> int:
-    import torch
+# A call costs its interpreter time: in a loop of small layers more than the kernels it enqueues. So the functions below
+# pack their argument structures in one go (filling a ctypes structure's 31 fields is 4 us, packing them 1 us), ask a tensor
+# for its strides once, and read the current stream's handle without making an object of it.
+_POOL = f"{ctypes.sizeof(PoolView)}s"
+_pack_decode = struct.Struct(f"@Pqq{_POOL}PqPPiiifPPPPPPNiiPqPqIPqPP").pack
+_pack_producer = struct.Struct(f"@{_POOL}PqPfPqPqPqPqqiPqPqP").pack
+_pack_indexer = struct.Struct("@PPPiPqPqPqPiiqiPPPNiP").pack
+for _pack, _type, _fields in ((_pack_decode, DecodeArgs, 31), (_pack_producer, ProducerArgs, 19), (_pack_indexer, IndexerArgs, 21)):
+    assert len(_pack(*(bytes(ctypes.sizeof(PoolView)) if t is PoolView else 0 for _, t in _type._fields_))) == ctypes.sizeof(_type)
+_torch_c = None
 
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return int(s.cuda_stream)
+
+def _stream_handle(stream=None) -> int:
+    global _torch_c
+    if stream is not None:
+        return stream.cuda_stream
+    if _torch_c is None:
+        import torch
+
+        torch.cuda.init()
+        _torch_c = torch._C
+    return _torch_c._cuda_getCurrentRawStream(_torch_c._cuda_getDevice())
 
 
 def _ptr(t) -> int:
-    return 0 if t is None else int(t.data_ptr())
+    return 0 if t is None else t.data_ptr()
 
 
 def pool_view(latent, rope=None) -> PoolView:
@@ -254,9 +272,9 @@ def new_status(device="cuda"):
 def append(view: PoolView, latent_src, rope_src, slot_mapping, status=None, stream=None) -> None:
     """latent_src bf16 [T, >=512] and rope_src bf16 [T, >=64] (row strides taken from the tensors),
     slot_mapping int32 [T] on the device."""
-    n = int(slot_mapping.shape[0])
-    check(lib.b200kv_append(ctypes.byref(view), _ptr(latent_src), latent_src.stride(0) if n else LATENT_DIM,
-                            _ptr(rope_src), rope_src.stride(0) if n else ROPE_DIM, _ptr(slot_mapping), n,
+    n = slot_mapping.shape[0]
+    check(lib.b200kv_append(ctypes.byref(view), latent_src.data_ptr(), latent_src.stride()[0] if n else LATENT_DIM,
+                            rope_src.data_ptr(), rope_src.stride()[0] if n else ROPE_DIM, slot_mapping.data_ptr(), n,
                             _stream_handle(stream), _ptr(status)))
 
 
@@ -266,39 +284,36 @@ def append_fused(view: PoolView, kv_a, gamma, cos, sin, slot_mapping, eps: float
     gamma bf16 [512], cos / sin bf16 [T, 64] (or [64] shared by all tokens), slot_mapping int32 [T].
     q_rope bf16 [T, heads, 64] is rotated in place; latent_out [T, 512], rope_out [T, 64] and rstd_out fp32
     [T] receive copies of what was computed."""
-    n = int(slot_mapping.shape[0])
-    a = ProducerArgs()
-    a.pool = view
-    a.kv_a, a.kv_a_stride = _ptr(kv_a), kv_a.stride(0) if n else LATENT_DIM + ROPE_DIM
-    a.gamma, a.eps = _ptr(gamma), eps
-    a.cos, a.cos_stride = _ptr(cos), (cos.stride(0) if cos.dim() == 2 else 0)
-    a.sin, a.sin_stride = _ptr(sin), (sin.stride(0) if sin.dim() == 2 else 0)
-    a.slot_mapping, a.n_tokens = _ptr(slot_mapping), n
+    n = slot_mapping.shape[0]
+    q_ptr = q_token_stride = q_head_stride = heads = 0
     if q_rope is not None:
-        a.q_rope, a.q_token_stride, a.q_head_stride, a.heads = _ptr(q_rope), q_rope.stride(0), q_rope.stride(1), \
-            int(q_rope.shape[1])
-    if latent_out is not None:
-        a.latent_out, a.latent_out_stride = _ptr(latent_out), latent_out.stride(0)
-    if rope_out is not None:
-        a.rope_out, a.rope_out_stride = _ptr(rope_out), rope_out.stride(0)
-    a.rstd_out = _ptr(rstd_out)
-    check(lib.b200kv_append_fused(ctypes.byref(a), _stream_handle(stream), _ptr(status)))
+        q_ptr, heads = q_rope.data_ptr(), q_rope.shape[1]
+        q_token_stride, q_head_stride = q_rope.stride()[:2]
+    latent_ptr, latent_stride = (0, 0) if latent_out is None else (latent_out.data_ptr(), latent_out.stride()[0])
+    rope_ptr, rope_stride = (0, 0) if rope_out is None else (rope_out.data_ptr(), rope_out.stride()[0])
+    cos_stride, sin_stride = cos.stride(), sin.stride()
+    a = _pack_producer(bytes(view), kv_a.data_ptr(), kv_a.stride()[0] if n else LATENT_DIM + ROPE_DIM, gamma.data_ptr(), eps,
+                     cos.data_ptr(), cos_stride[0] if len(cos_stride) == 2 else 0,
+                     sin.data_ptr(), sin_stride[0] if len(sin_stride) == 2 else 0, slot_mapping.data_ptr(), n,
+                     q_ptr, q_token_stride, q_head_stride, heads, latent_ptr, latent_stride, rope_ptr, rope_stride,
+                     _ptr(rstd_out))
+    check(lib.b200kv_append_fused(a, _stream_handle(stream), _ptr(status)))
 
 
 def mx_quant_e4m3(x, q, scales, stream=None) -> None:
     """x bf16 [rows, cols] -> q uint8 [rows, cols] (FP8 E4M3 codes), scales uint8 [rows, cols / 32] (E8M0)."""
-    rows, cols = int(x.shape[0]), int(x.shape[1])
-    check(lib.b200kv_mx_quant_e4m3(_ptr(x), x.stride(0), rows, cols, _ptr(q), q.stride(0), _ptr(scales),
-                                   scales.stride(0), _stream_handle(stream)))
+    rows, cols = x.shape
+    check(lib.b200kv_mx_quant_e4m3(x.data_ptr(), x.stride()[0], rows, cols, q.data_ptr(), q.stride()[0], scales.data_ptr(),
+                                   scales.stride()[0], _stream_handle(stream)))
 
 
 def gather(view: PoolView, block_table, kv_len, block_size: int, out_latent, out_rope, out_row_offsets,
            total_rows: int, status=None, stream=None) -> None:
-    batch = int(kv_len.shape[0])
-    check(lib.b200kv_gather(ctypes.byref(view), _ptr(block_table), block_table.stride(0) if batch else 1,
-                            _ptr(kv_len), batch, block_size, _ptr(out_latent),
-                            out_latent.stride(0) if total_rows else LATENT_DIM, _ptr(out_rope),
-                            out_rope.stride(0) if total_rows else ROPE_DIM, _ptr(out_row_offsets), total_rows,
+    batch = kv_len.shape[0]
+    check(lib.b200kv_gather(ctypes.byref(view), block_table.data_ptr(), block_table.stride()[0] if batch else 1,
+                            kv_len.data_ptr(), batch, block_size, out_latent.data_ptr(),
+                            out_latent.stride()[0] if total_rows else LATENT_DIM, out_rope.data_ptr(),
+                            out_rope.stride()[0] if total_rows else ROPE_DIM, out_row_offsets.data_ptr(), total_rows,
                             _stream_handle(stream), _ptr(status)))
 
 
@@ -311,19 +326,15 @@ def indexer_topk(q_fp8, q_scale, weights, key_pool, k_scale, block_table, kv_len
     rows_out int32 [B, k]: also receives the selection as pool rows (see resolve_rows)."""
     import torch
 
-    batch, heads = int(q_fp8.shape[0]), int(q_fp8.shape[1])
+    batch, heads = q_fp8.shape[:2]
     index = torch.empty((batch, k), dtype=torch.int32, device=q_fp8.device)
     n_sel = torch.empty((batch,), dtype=torch.int32, device=q_fp8.device)
     ws = torch.empty(lib.b200kv_indexer_workspace_bytes(batch, max_kv_len), dtype=torch.uint8, device=q_fp8.device)
-    a = IndexerArgs()
-    a.q, a.q_scale, a.weights, a.heads = _ptr(q_fp8), _ptr(q_scale), _ptr(weights), heads
-    a.key_pool, a.key_stride, a.k_scale, a.pool_rows = _ptr(key_pool), key_pool.stride(0), _ptr(k_scale), key_pool.shape[0]
-    a.block_table, a.max_blocks, a.kv_len = _ptr(block_table), block_table.shape[1], _ptr(kv_len)
-    a.batch, a.block_size, a.max_kv_len, a.k = batch, block_size, max_kv_len, k
-    a.index_out, a.n_selected_out, a.workspace, a.workspace_bytes = _ptr(index), _ptr(n_sel), _ptr(ws), ws.numel()
-    a.variant = variant
-    a.rows_out = _ptr(rows_out)
-    check(lib.b200kv_indexer_topk(ctypes.byref(a), _stream_handle(stream), _ptr(status)))
+    a = _pack_indexer(q_fp8.data_ptr(), q_scale.data_ptr(), weights.data_ptr(), heads, key_pool.data_ptr(), key_pool.stride()[0],
+                    k_scale.data_ptr(), key_pool.shape[0], block_table.data_ptr(), block_table.shape[1], kv_len.data_ptr(),
+                    batch, block_size, max_kv_len, k, index.data_ptr(), n_sel.data_ptr(), ws.data_ptr(), ws.numel(), variant,
+                    _ptr(rows_out))
+    check(lib.b200kv_indexer_topk(a, _stream_handle(stream), _ptr(status)))
     if scores_out is not None:
         stride = (max_kv_len + 3) & ~3  # the scores lie first in the workspace, [batch][stride] fp32
         scores_out.append(ws[: batch * stride * 4].view(torch.float32).view(batch, stride))
@@ -359,61 +370,30 @@ def mla_decode(q, view: PoolView, block_table, kv_len, block_size: int, scale: f
     row_index int32 [B, max_selected]: attend over these pool rows (kv_len = how many per sequence) instead of the
     block table, which may then be None. quantised = (fp8 uint8 [B, H, 512], scales uint8 [B, H, 16]): the output's MX
     quantisation written by the same launch."""
-    args = DecodeArgs()
-    args.q = _ptr(q)
-    args.q_seq_stride = q.stride(0)
-    args.q_head_stride = q.stride(1)
-    args.pool = view
-    args.block_table = _ptr(block_table)
-    args.max_blocks = 0 if block_table is None else block_table.stride(0)
-    if row_index is not None:
-        args.row_index, args.row_index_stride = _ptr(row_index), row_index.stride(0)
-    if quantised is not None:
-        args.out_fp8, args.out_scale = _ptr(quantised[0]), _ptr(quantised[1])
-    args.kv_len = _ptr(kv_len)
-    args.kv_begin = _ptr(kv_begin)
-    args.batch = q.shape[0]
-    args.heads = q.shape[1]
-    args.block_size = block_size
-    args.scale = scale
-    args.out = _ptr(out)
-    args.lse = _ptr(lse)
-    if partial is not None:
-        args.partial_o, args.partial_m, args.partial_l = (_ptr(t) for t in partial)
-    args.workspace = _ptr(workspace)
-    args.workspace_bytes = 0 if workspace is None else workspace.numel() * workspace.element_size()
-    args.variant = variant
-    args.max_ctas = max_ctas
-    args.flags = 1 if stable_tables else 0
-    if new_rows is not None:
-        new_latent, new_rope = new_rows
-        args.new_latent, args.new_latent_stride = _ptr(new_latent), new_latent.stride(0)
-        args.new_rope, args.new_rope_stride = _ptr(new_rope), new_rope.stride(0)
-    check(lib.b200kv_mla_decode(ctypes.byref(args), _stream_handle(stream), _ptr(status)))
+    args = _decode_args(q, view, block_table, kv_len, block_size, scale, out, lse, kv_begin, workspace, max_ctas, stable_tables,
+                        partial, variant, new_rows, row_index, quantised)
+    check(lib.b200kv_mla_decode(args, _stream_handle(stream), _ptr(status)))
 
 
 def _decode_args(q, view: PoolView, block_table, kv_len, block_size: int, scale: float, out=None, lse=None, kv_begin=None,
-                 workspace=None, max_ctas: int = 0, stable_tables: bool = False) -> DecodeArgs:
-    args = DecodeArgs()
-    args.q = _ptr(q)
-    args.q_seq_stride = q.stride(0)
-    args.q_head_stride = q.stride(1)
-    args.pool = view
-    args.block_table = _ptr(block_table)
-    args.max_blocks = block_table.stride(0)
-    args.kv_len = _ptr(kv_len)
-    args.kv_begin = _ptr(kv_begin)
-    args.batch = q.shape[0]
-    args.heads = q.shape[1]
-    args.block_size = block_size
-    args.scale = scale
-    args.out = _ptr(out)
-    args.lse = _ptr(lse)
-    args.workspace = _ptr(workspace)
-    args.workspace_bytes = 0 if workspace is None else workspace.numel() * workspace.element_size()
-    args.max_ctas = max_ctas
-    args.flags = 1 if stable_tables else 0
-    return args
+                 workspace=None, max_ctas: int = 0, stable_tables: bool = False, partial=None, variant: int = DECODE_AUTO,
+                 new_rows=None, row_index=None, quantised=None) -> bytes:
+    """b200kv_decode_args, packed."""
+    batch, heads = q.shape[:2]
+    q_seq_stride, q_head_stride = q.stride()[:2]
+    table, max_blocks = (0, 0) if block_table is None else (block_table.data_ptr(), block_table.stride()[0])
+    o, m, l = (0, 0, 0) if partial is None else (_ptr(partial[0]), _ptr(partial[1]), _ptr(partial[2]))
+    ws, ws_bytes = (0, 0) if workspace is None else (workspace.data_ptr(), workspace.nbytes)
+    if new_rows is None:
+        latent = latent_stride = rope = rope_stride = 0
+    else:
+        latent, latent_stride = new_rows[0].data_ptr(), new_rows[0].stride()[0]
+        rope, rope_stride = new_rows[1].data_ptr(), new_rows[1].stride()[0]
+    rows, rows_stride = (0, 0) if row_index is None else (row_index.data_ptr(), row_index.stride()[0])
+    fp8, scales = (0, 0) if quantised is None else (_ptr(quantised[0]), _ptr(quantised[1]))
+    return _pack_decode(q.data_ptr(), q_seq_stride, q_head_stride, bytes(view), table, max_blocks, kv_len.data_ptr(), _ptr(kv_begin),
+                      batch, heads, block_size, scale, _ptr(out), _ptr(lse), o, m, l, ws, ws_bytes, variant, max_ctas,
+                      latent, latent_stride, rope, rope_stride, 1 if stable_tables else 0, rows, rows_stride, fp8, scales)
 
 
 def mla_decode_static(q, view: PoolView, block_table, kv_len, block_size: int, scale: float, out=None, lse=None,
@@ -421,31 +401,14 @@ def mla_decode_static(q, view: PoolView, block_table, kv_len, block_size: int, s
     """b200kv_mla_decode_static: the same attention, with the library's built-in scratch instead of a
     workspace tensor; nothing is allocated on the device by the call."""
     lib.b200kv_mla_decode_static.restype = c_int32
-    lib.b200kv_mla_decode_static.argtypes = [POINTER(DecodeArgs), c_void_p, c_void_p]
-    args = DecodeArgs()
-    args.q = _ptr(q)
-    args.q_seq_stride = q.stride(0)
-    args.q_head_stride = q.stride(1)
-    args.pool = view
-    args.block_table = _ptr(block_table)
-    args.max_blocks = block_table.stride(0)
-    args.kv_len = _ptr(kv_len)
-    args.kv_begin = _ptr(kv_begin)
-    args.batch = q.shape[0]
-    args.heads = q.shape[1]
-    args.block_size = block_size
-    args.scale = scale
-    args.out = _ptr(out)
-    args.lse = _ptr(lse)
-    if partial is not None:
-        args.partial_o, args.partial_m, args.partial_l = (_ptr(t) for t in partial)
-    args.max_ctas = max_ctas
-    check(lib.b200kv_mla_decode_static(ctypes.byref(args), _stream_handle(stream), _ptr(status)))
+    lib.b200kv_mla_decode_static.argtypes = [c_void_p, c_void_p, c_void_p]
+    args = _decode_args(q, view, block_table, kv_len, block_size, scale, out, lse, kv_begin, None, max_ctas, False, partial)
+    check(lib.b200kv_mla_decode_static(args, _stream_handle(stream), _ptr(status)))
 
 
 def lse_merge(partial_o, partial_m, partial_l, out, lse=None, stream=None) -> None:
     """partial_o fp32 [P, rows, 512], partial_m / partial_l fp32 [P, rows] -> out bf16 [rows, 512]."""
-    n_parts, rows = int(partial_m.shape[0]), int(partial_m.shape[1])
+    n_parts, rows = partial_m.shape
     check(lib.b200kv_lse_merge(_ptr(partial_o), _ptr(partial_m), _ptr(partial_l), n_parts, rows, _ptr(out),
                                _ptr(lse), _stream_handle(stream)))
 
@@ -773,13 +736,16 @@ class Engine:
                                            _stream_handle(stream) if self.config.backend == 0 else None))
 
     def layer_append(self, layer: int, kv_a, gamma, cos, sin, q_rope=None, stream=None):
+        cos_stride, sin_stride = cos.stride(), sin.stride()
+        q_ptr, q_stride = (0, (0, 0)) if q_rope is None else (q_rope.data_ptr(), q_rope.stride())
         check(lib.b200kv_engine_layer_append(
-            self._h, layer, _ptr(kv_a), kv_a.stride(0), _ptr(gamma), _ptr(cos), cos.stride(0) if cos.dim() == 2 else 0,
-            _ptr(sin), sin.stride(0) if sin.dim() == 2 else 0, _ptr(q_rope),
-            0 if q_rope is None else q_rope.stride(0), 0 if q_rope is None else q_rope.stride(1), _stream_handle(stream)))
+            self._h, layer, kv_a.data_ptr(), kv_a.stride()[0], gamma.data_ptr(), cos.data_ptr(),
+            cos_stride[0] if len(cos_stride) == 2 else 0, sin.data_ptr(), sin_stride[0] if len(sin_stride) == 2 else 0,
+            q_ptr, q_stride[0], q_stride[1], _stream_handle(stream)))
 
     def layer_attend(self, layer: int, q, out, out_fp8=None, out_scales=None, stream=None):
-        check(lib.b200kv_engine_layer_attend(self._h, layer, _ptr(q), q.stride(0), q.stride(1), _ptr(out), _ptr(out_fp8),
+        q_stride = q.stride()
+        check(lib.b200kv_engine_layer_attend(self._h, layer, q.data_ptr(), q_stride[0], q_stride[1], _ptr(out), _ptr(out_fp8),
                                              _ptr(out_scales), _stream_handle(stream)))
 
     def end_step(self):

@@ -133,7 +133,7 @@ class PeerExchange:
 
         args = _decode_args(q, view, block_table, kv_len, block_size, scale, out=out, lse=lse, kv_begin=kv_begin,
                             workspace=workspace, max_ctas=max_ctas, stable_tables=stable_tables)
-        check(lib.b200kv_mla_decode_peer(ctypes.byref(args), self._table, self.world, self.rank,
+        check(lib.b200kv_mla_decode_peer(args, self._table, self.world, self.rank,
                                          _stream_handle(stream), _ptr(status)))
         return out
 
