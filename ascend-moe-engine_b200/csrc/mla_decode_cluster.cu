@@ -133,12 +133,13 @@ struct Share {
   int first_peer;    // cluster rank of the first CTA of the same heads
 };
 
-__device__ __forceinline__ Share ShareOf(int tiles, int cluster, int rank, int group_heads) {
+// one_tile: no CTA is to have more than one tile, if there are CTAs enough.
+__device__ __forceinline__ Share ShareOf(int tiles, int cluster, int rank, int group_heads, bool one_tile) {
   int log2 = 31 - __clz(cluster), heads = group_heads;
   // Halving the ranges halves what a CTA sends (64 KB at 64 heads and some 30 bytes a cycle) and the heads of Q it loads,
   // and adds tiles (72 KB at 27 bytes a cycle): worth it while it adds none, and from 64 heads also for the second tile
   // of some CTAs (one sequence of 1,024 tokens: 16.1 us in 16 ranges, 12.9 us in 8).
-  while (heads > kLeastHeads && log2 > 0 && (2 * tiles <= (1 << log2) || (heads == kHeads && 2 * tiles <= (3 << log2)))) {
+  while (heads > kLeastHeads && log2 > 0 && (2 * tiles <= (1 << log2) || (!one_tile && heads == kHeads && 2 * tiles <= (3 << log2)))) {
     --log2;
     heads >>= 1;
   }
@@ -253,7 +254,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   }
   const int len = max(p.kv_len[seq], 0);
   const int begin = p.kv_begin ? p.kv_begin[seq] : 0;
-  const Share share = ShareOf(TilesOf(len), cluster, rank, p.group_heads);
+  const Share share = ShareOf(TilesOf(len), cluster, rank, p.group_heads, p.out_q != nullptr);
   const int n = share.t_hi - share.t_lo;
   const bool appends = p.new_latent != nullptr && n > 0 && share.t_hi == TilesOf(len);  // the new row is in this CTA's last tile
   int64_t first_row = 0;
@@ -1146,6 +1147,10 @@ int32_t TryDecodeCluster(const b200kv_decode_args& a, cudaStream_t stream, int32
   const int64_t most_tiles = a.row_index != nullptr ? (a.row_index_stride + kTile - 1) / kTile
                                                     : a.max_blocks * ((a.block_size + kTile - 1) / kTile);
   if (most_tiles > MostTilesFor(cluster, a.batch)) return B200KV_OK;
+  // The weights are rounded to bf16 against the maximum of a CTA's first tile, so which tiles share a CTA moves results by
+  // roundings: nothing in a bf16 row, but one in a hundred of its FP8 codes. Quantised calls keep their bytes: they come
+  // here only where every tile has a CTA and a maximum of its own, as the flat kernel has it for so few tiles.
+  if (a.out_fp8 != nullptr && most_tiles > cluster) return B200KV_OK;
   *launched = true;
   return Launch(a, a.row_index != nullptr ? kRowList : kTiles, false, cluster, kHeads, stream, status);
 }
