@@ -259,7 +259,7 @@ def test_indexer_selection_matches_oracle_bit_for_bit(lens, k):
     assert np.array_equal(index.cpu().numpy(), exp_index), "selection differs from the oracle"
 
 
-@pytest.mark.parametrize("length", [500, 4096, 5000, 20000, 70000, 150000])
+@pytest.mark.parametrize("length", [128, 129, 500, 4096, 5000, 20000, 70000, 150000])
 @pytest.mark.parametrize("shape", ["equal", "outlier", "two values"])
 def test_indexer_selection_of_scores_that_bins_do_not_separate(length, shape):
     """All scores equal (positions decide, in passes down to single positions), one score a million times the others
