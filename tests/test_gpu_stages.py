@@ -284,6 +284,7 @@ def test_indexer_selection_of_scores_that_bins_do_not_separate(length, shape):
     index, n = b200kv.indexer_topk(q, one, one.bfloat16(), key, ks, table, to_dev_i32([length]), bs, length, k,
                                    variant=b200kv.INDEXER_EXACT)
     want = torch.sort(ks[:length].cpu(), descending=True, stable=True).indices[:k]
+    want = torch.cat([want, torch.full((k - len(want),), -1)])
     assert int(n[0]) == min(k, length)
     assert torch.equal(index[0].cpu().long(), want)
 
