@@ -1,6 +1,8 @@
 """The stages beside the KV path on the GPU, through the C ABI: the fused producer (RMSNorm + rotary
 embedding + paged write, and the query's rope slices) and the MX quantiser of the attention output.
 Their arithmetic is fixed to the operation, so everything is compared bit for bit with the oracle."""
+from ctypes import c_int32, c_int64, c_void_p
+
 import numpy as np
 import pytest
 import torch
@@ -472,3 +474,30 @@ def test_indexer_operator_through_the_operator_abi():
     got = out.cpu().numpy()[:, 0, :]
     _check_selection_up_to_rounding(got, (got >= 0).sum(axis=1).astype(np.int32), None, exp_scores, exp_n, kv_len, k,
                                     eps_rel=1e-6)
+
+
+@pytest.mark.parametrize("tokens,heads", [(31, 63), (593, 64), (1025, 64), (1203, 63), (2, 5000)])
+def test_query_rotation_in_its_own_kernel(tokens, heads):
+    """Query slices that share the rows' launch and those that get their own (from four passes a warp on), with one and
+    two rounds a warp, on both sides of each line; slices of wider rows, so that the rest has to stay as it is."""
+    rows = tokens + 64
+    kv_a = kvo.normal_bf16(tokens * 576, 3).reshape(tokens, 576)
+    gamma, (cos, sin) = gamma_bits(), rope_tables(tokens, first_pos=11)
+    slots = kvo.permutation(rows)[:tokens].astype(np.int32)
+    q = kvo.normal_bf16(tokens * heads * 72, 2).reshape(tokens, heads, 72)
+    expect_q = q.copy()
+    expect_q[:, :, 8:] = kvo.rope_half64(np.ascontiguousarray(q[:, :, 8:]), cos, sin)
+    expect = np.zeros((rows, 576), dtype=np.uint16)
+    kvo.append_fused(expect, kv_a, gamma, cos, sin, slots)
+    pool = torch.zeros((rows, 576), dtype=torch.bfloat16, device="cuda")
+    d_q, d_cos, d_sin = to_dev_bf16(q), to_dev_bf16(cos), to_dev_bf16(sin)
+    b200kv.append_fused(b200kv.pool_view(pool), to_dev_bf16(kv_a), to_dev_bf16(gamma), d_cos, d_sin, to_dev_i32(slots),
+                        q_rope=d_q[:, :, 8:])
+    assert np.array_equal(from_dev_bf16(d_q), expect_q)
+    assert np.array_equal(from_dev_bf16(pool), expect)
+    d_q = to_dev_bf16(q)  # and without rows
+    rotate = b200kv.lib.b200kv_rope_half64
+    rotate.argtypes = [c_void_p, c_int64, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_int64, c_int32, c_void_p]
+    assert rotate(d_q.data_ptr() + 16, heads * 72, 72, d_cos.data_ptr(), 64, d_sin.data_ptr(), 64, tokens, heads,
+                  torch.cuda.current_stream().cuda_stream) == 0
+    assert np.array_equal(from_dev_bf16(d_q), expect_q)
