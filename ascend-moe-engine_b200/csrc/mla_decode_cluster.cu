@@ -27,7 +27,8 @@
 //
 // Roles as in the flat kernel: warps 0-3 softmax, 4 producer, 5 QK, 6 PV; all eight warps take part in the exchange and
 // the merge. Every wait is bounded; a CTA
-// that gives up still arrives at the cluster barriers, so no peer is left waiting.
+// that gives up still arrives at the cluster barriers, so no peer is left waiting. The softmax warps share barriers that
+// have no bound, so they give up together (see the loop).
 #include <cuda.h>
 #include <cuda_fp8.h>
 
@@ -578,11 +579,14 @@ __global__ void __launch_bounds__(kThreads, 1)
     const int head0 = warp * 16 + quad_row;  // and head0 + 8: this thread's two rows
     const uint32_t lane_base = static_cast<uint32_t>(warp * 32) << 16;
     const bool has_rows = warp * 16 < share.heads;  // otherwise the warp only keeps step with the others
+    // The four warps leave the loop on the same tile: a wait can run out for one of them and not for another, and whoever
+    // stayed would stand at the named barriers for good. So a warp whose wait ran out goes on, with whatever the
+    // accumulators hold (the result is void), asks for the rescaling path, and there all four leave on one vote. The usual
+    // path carries no vote of its own.
     for (int i = 0; i < n; ++i) {
       const int buf = kSplitP ? 0 : i & 1, stage = i % kStages;
       const int valid = min(kTile, len - (share.t_lo + i) * kTile);
-      ok = WarpWait(bar(&misc->s_full[buf]), (kSplitP ? i : i >> 1) & 1, misc, p.status, 230);
-      if (!ok) break;
+      if (ok) ok = WarpWait(bar(&misc->s_full[buf]), (kSplitP ? i : i >> 1) & 1, misc, p.status, 230);
       ptx::TcFenceAfterSync();
       uint32_t sr[32];
       if (has_rows) {
@@ -663,15 +667,18 @@ __global__ void __launch_bounds__(kThreads, 1)
         sum += __shfl_xor_sync(0xffffffffu, sum, 2);
         l_run[r] += sum;
       }
-      const bool any_rescale = ptx::NamedBarrierOr(1, kSoftmaxThreads, rescale);
-      if (i > 0 && (any_rescale || kSplitP)) {
+      const bool any_rescale = ptx::NamedBarrierOr(1, kSoftmaxThreads, rescale || !ok);
+      if (ok && i > 0 && (any_rescale || kSplitP)) {
         // PV of the previous tile must have drained: before its accumulators are rescaled (rare), and before the one
         // buffer of P's low term is written again. (It ran under this tile's exponentials.)
         ok = WarpWait(bar(&misc->kv_empty[(i - 1) % kStages][kGroups - 1]), ((i - 1) / kStages) & 1, misc, p.status, 231);
-        if (!ok) break;
         ptx::TcFenceAfterSync();
       }
       if (any_rescale) {
+        if (ptx::NamedBarrierOr(2, kSoftmaxThreads, !ok)) {
+          ok = false;
+          break;
+        }
 #pragma unroll 1
         for (int tm = 0; tm < 4; ++tm) {
 #pragma unroll 1
