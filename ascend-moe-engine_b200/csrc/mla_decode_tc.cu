@@ -804,13 +804,15 @@ __global__ void __launch_bounds__(kThreads, 1)
       float m_run[2] = {-INFINITY, -INFINITY};  // reference maxima of the two rows, log2 domain (s * scale * log2e)
       float l_run[2] = {0.0f, 0.0f};
       const int n = t_hi - t_lo;
-      for (int i = 0; i < n && ok; ++i, ++g) {
+      // The four warps leave this loop, and the segment, on the same vote: a wait can run out for one of them and not for
+      // another, and whoever stayed would stand at the named barriers for good. A warp whose wait for S ran out goes on,
+      // with whatever the accumulator holds (the result is void), and asks for the rescaling path, where the vote is.
+      for (int i = 0; i < n; ++i, ++g) {
         const int buf = g & 1;
         const int stage = g % kStages;
         const int tok0 = (t_lo + i) * kTile;
         const int valid = min(kTile, seq_len - tok0);
-        ok = BoundedWait(bar(&misc->s_full[buf]), (g >> 1) & 1, misc, p.status, 30);
-        if (!ok) break;
+        ok = __all_sync(0xffffffffu, BoundedWait(bar(&misc->s_full[buf]), (g >> 1) & 1, misc, p.status, 30));
         ptx::TcFenceAfterSync();
         static_assert(kTile == 64, "one 16x256b.x8 load covers the 64 columns of a tile");
         uint32_t sr[32];
@@ -884,13 +886,20 @@ __global__ void __launch_bounds__(kThreads, 1)
           l_run[r] += sum;
         }
 
-        const bool any_rescale = ptx::NamedBarrierOr(1, kSoftmaxThreads, rescale);
+        const bool any_rescale = ptx::NamedBarrierOr(1, kSoftmaxThreads, rescale || !ok);
         if (any_rescale) {
           // Rare path: scale the accumulated O^T columns (heads) by their factors. PV of the previous
-          // tile must have drained first; its commit is the arrival on that tile's kv_empty.
+          // tile must have drained first; its commit is the arrival on that tile's kv_empty. (A segment's first tile
+          // comes here only to give up: there is no tile before it to wait for.)
           const int gp = g - 1;
-          ok = BoundedWait(bar(&misc->kv_empty[gp % kStages][kGroups - 1]), (gp / kStages) & 1, misc, p.status, 31);
-          if (!ok) break;
+          if (ok && i > 0) {
+            ok = __all_sync(0xffffffffu,
+                            BoundedWait(bar(&misc->kv_empty[gp % kStages][kGroups - 1]), (gp / kStages) & 1, misc, p.status, 31));
+          }
+          if (ptx::NamedBarrierOr(2, kSoftmaxThreads, !ok)) {
+            ok = false;
+            break;
+          }
           ptx::TcFenceAfterSync();
 #pragma unroll 1
           for (int tm = 0; tm < 4; ++tm) {
@@ -942,8 +951,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       if (!ok) break;
 
       // ---- epilogue of the segment ----
-      ok = BoundedWait(bar(&misc->o_full), seg & 1, misc, p.status, 32);
-      if (!ok) break;
+      ok = __all_sync(0xffffffffu, BoundedWait(bar(&misc->o_full), seg & 1, misc, p.status, 32));
       ptx::TcFenceAfterSync();
       const bool whole = (t_lo == 0 && t_hi == seq_tiles);
       const bool to_ws = !whole || p.force_ws != 0;
@@ -967,7 +975,10 @@ __global__ void __launch_bounds__(kThreads, 1)
           p.lse[static_cast<int64_t>(seq) * kHeads + head] = m_nat + logf(l_row);
         }
       }
-      ptx::NamedBarrier(1, kSoftmaxThreads);
+      if (ptx::NamedBarrierOr(1, kSoftmaxThreads, !ok)) {
+        ok = false;
+        break;
+      }
       if (to_ws) {
         // The usual case (a sequence cut over several CTAs). Both halves of an accumulator are read before the
         // one wait; store j of a warp is the 512 contiguous bytes of head quad j, dv 32 w .. 32 w + 31.

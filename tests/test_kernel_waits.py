@@ -12,6 +12,7 @@ CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))),
 # file, first and last text of the role whose warps share barriers
 ROLES = {
     "mla_decode_cluster.cu": ("= softmax =", "if (warp == 5 || warp == 6)"),
+    "mla_decode_tc.cu": ("= softmax + epilogue warps =", "// ---- teardown"),
 }
 
 EVENT = re.compile(
