@@ -341,16 +341,18 @@ __global__ void __launch_bounds__(kThreads, 1)
     bool have = fetch(&next);
     bool ok = true;
     const int buf = group;
-    for (int n = 0; ok && have; ++n) {  // the group's n-th tile is the run's tile 2 n + group
+    // (The group's warps leave on the same tile, by the barrier's vote: a wait can run out for one of them and not for
+    // another, and whoever stayed would stand at the barrier for good. A warp whose wait ran out finishes its tile with
+    // whatever the accumulator holds; the result is void.)
+    for (int n = 0; have; ++n) {  // the group's n-th tile is the run's tile 2 n + group
       cur = next;
       have = fetch(&next);
       if (gtid < kHeadsPadded) {
         sh->qs[buf][n & 1][gtid] = cur.qs;
         sh->w[buf][n & 1][gtid] = cur.w;
       }
-      ptx::NamedBarrier(1 + group, kEpilogueThreads);
+      if (ptx::NamedBarrierOr(1 + group, kEpilogueThreads, !ok)) break;
       ok = __all_sync(0xffffffffu, Wait(bar(&sh->acc_full[buf]), n & 1, sh, p.status, 3));
-      if (!ok) break;
       ptx::TcFenceAfterSync();
       uint32_t lo[32], hi[32];
       const uint32_t taddr = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16) + buf * kHeadsPadded;

@@ -13,6 +13,7 @@ CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))),
 ROLES = {
     "mla_decode_cluster.cu": ("= softmax =", "if (warp == 5 || warp == 6)"),
     "mla_decode_tc.cu": ("= softmax + epilogue warps =", "// ---- teardown"),
+    "kv_indexer_tc.cu": ("// ---- epilogue: thread = token", "TmemDealloc"),
 }
 
 EVENT = re.compile(
