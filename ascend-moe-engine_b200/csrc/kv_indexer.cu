@@ -167,6 +167,7 @@ struct SelectParams {
   int32_t block_size;
   int64_t pool_rows;
   int32_t* rows_out;    // [batch][k] or null
+  int32_t cluster_log2; // of the CTAs that take a sequence
   int32_t* status;
 };
 
@@ -243,8 +244,8 @@ __global__ void __launch_bounds__(kSortThreads) IndexerSelectKernel(SelectParams
   SelectShared& sh = *reinterpret_cast<SelectShared*>(select_smem);
   GridDependencyTrigger();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int cluster = gridDim.x, rank = blockIdx.x, b = blockIdx.y;
-  const int cluster_log2 = 31 - __clz(cluster);
+  const int cluster_log2 = p.cluster_log2, cluster = 1 << cluster_log2;
+  const int rank = blockIdx.x & (cluster - 1), b = blockIdx.x >> cluster_log2;
   auto cluster_sync = [&]() {
     if (cluster > 1) {
       __syncwarp();
@@ -535,7 +536,7 @@ __global__ void __launch_bounds__(kSortThreads) IndexerSelectKernel(SelectParams
   for (int i = tid; i < kept; i += kSortThreads) write(sh.all[i], i);
 }
 
-int32_t LaunchSelect(const SelectParams& p, int32_t batch, int64_t max_kv_len, cudaStream_t stream) {
+int32_t LaunchSelect(SelectParams p, int32_t batch, int64_t max_kv_len, cudaStream_t stream) {
   // How many clusters of 1, 2, 4, 8, 16 CTAs the device holds at once; looked up once per thread and device.
   static thread_local int known_device = -1;
   static thread_local int32_t most[5];
@@ -571,8 +572,9 @@ int32_t LaunchSelect(const SelectParams& p, int32_t batch, int64_t max_kv_len, c
   int size = 0;
   while (size < 4 && max_kv_len > static_cast<int64_t>(kTokensPerCta) << size) ++size;
   while (size > 0 && batch > most[size]) --size;
+  p.cluster_log2 = size;
   attrs[0].val.clusterDim.x = 1u << size;
-  config.gridDim = dim3(1u << size, static_cast<unsigned>(batch));
+  config.gridDim = dim3(static_cast<unsigned>(batch) << size);  // (in x, which has room for any batch)
   config.numAttrs = 2;
   return CheckCuda(cudaLaunchKernelEx(&config, IndexerSelectKernel, p), "indexer top-k launch");
 }

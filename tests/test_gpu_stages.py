@@ -261,6 +261,28 @@ def test_indexer_selection_matches_oracle_bit_for_bit(lens, k):
     assert np.array_equal(index.cpu().numpy(), exp_index), "selection differs from the oracle"
 
 
+def test_indexer_selection_of_more_sequences_than_a_grid_is_high():
+    """65,600 sequences of one to three tokens: the batch exceeds what a grid's second and third extents can hold."""
+    B, bs, k = 65600, 64, 2
+    g = torch.Generator(device="cuda")
+    g.manual_seed(5)
+    q = torch.randn((B, 1, 128), generator=g, device="cuda").to(torch.float8_e4m3fn).view(torch.uint8)
+    key = torch.randn((8 * bs, 128), generator=g, device="cuda").to(torch.float8_e4m3fn).view(torch.uint8)
+    w = torch.ones((B, 1), dtype=torch.bfloat16, device="cuda")
+    lens = torch.arange(B, device="cuda", dtype=torch.int32) % 3 + 1
+    table = (torch.arange(B, device="cuda", dtype=torch.int32) % 8).view(B, 1).contiguous()
+    st, scores = b200kv.new_status(), []
+    index, n_sel = b200kv.indexer_topk(q, torch.ones((B, 1), device="cuda"), w, key, torch.ones(8 * bs, device="cuda"), table, lens, bs, 3, k,
+                                       status=st, variant=b200kv.INDEXER_TCGEN05, scores_out=scores)
+    torch.cuda.synchronize()
+    assert st.cpu().tolist()[0] == 0
+    assert torch.equal(n_sel, lens.clamp(max=k))
+    masked = torch.where(torch.arange(4, device="cuda") < lens[:, None], scores[0], float("-inf"))
+    want = torch.sort(masked, dim=1, descending=True, stable=True)[1][:, :k].int()
+    want[torch.arange(k, device="cuda") >= n_sel[:, None]] = -1
+    assert torch.equal(index, want)
+
+
 @pytest.mark.parametrize("length", [128, 129, 500, 4096, 5000, 20000, 70000, 150000])
 @pytest.mark.parametrize("shape", ["equal", "outlier", "two values"])
 def test_indexer_selection_of_scores_that_bins_do_not_separate(length, shape):
