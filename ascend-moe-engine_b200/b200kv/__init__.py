@@ -143,16 +143,18 @@ def _load() -> ctypes.CDLL:
     lib.b200kv_mla_decode_workspace_bytes.restype = c_size_t
     lib.b200kv_mla_decode_workspace_bytes.argtypes = [c_int32, c_int32, c_int32]
     lib.b200kv_mla_decode.restype = c_int32
-    lib.b200kv_mla_decode.argtypes = [c_void_p, c_void_p, c_void_p]
+    lib.b200kv_mla_decode.argtypes = [POINTER(DecodeArgs), c_void_p, c_void_p]
+    lib.b200kv_mla_decode_static.restype = c_int32
+    lib.b200kv_mla_decode_static.argtypes = [POINTER(DecodeArgs), c_void_p, c_void_p]
     lib.b200kv_append_fused.restype = c_int32
-    lib.b200kv_append_fused.argtypes = [c_void_p, c_void_p, c_void_p]
+    lib.b200kv_append_fused.argtypes = [POINTER(ProducerArgs), c_void_p, c_void_p]
     lib.b200kv_mx_quant_e4m3.restype = c_int32
     lib.b200kv_mx_quant_e4m3.argtypes = [c_void_p, c_int64, c_int64, c_int64, c_void_p, c_int64, c_void_p, c_int64,
                                          c_void_p]
     lib.b200kv_indexer_workspace_bytes.restype = c_size_t
     lib.b200kv_indexer_workspace_bytes.argtypes = [c_int32, c_int64]
     lib.b200kv_indexer_topk.restype = c_int32
-    lib.b200kv_indexer_topk.argtypes = [c_void_p, c_void_p, c_void_p]
+    lib.b200kv_indexer_topk.argtypes = [POINTER(IndexerArgs), c_void_p, c_void_p]
     lib.b200kv_resolve_rows.restype = c_int32
     lib.b200kv_resolve_rows.argtypes = [c_void_p, c_int64, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_int64,
                                         c_void_p, c_void_p, c_void_p]
@@ -228,6 +230,24 @@ for _pack, _type, _fields in ((_pack_decode, DecodeArgs, 31), (_pack_producer, P
 _torch_c = None
 
 
+def _packed_entry(name: str):
+    """The entry point `name` for packed arguments: a function object of its own, so that `lib`'s keeps its argument types."""
+    fn = lib[name]
+    fn.restype = c_int32
+    fn.argtypes = [c_void_p, c_void_p, c_void_p]
+    return fn
+
+
+_mla_decode, _mla_decode_static = _packed_entry("b200kv_mla_decode"), _packed_entry("b200kv_mla_decode_static")
+_append_fused, _indexer_topk = _packed_entry("b200kv_append_fused"), _packed_entry("b200kv_indexer_topk")
+
+
+def _view_bytes(view: PoolView) -> bytes:
+    if not isinstance(view, PoolView):
+        raise TypeError(f"expected a PoolView, got {type(view).__name__}")
+    return bytes(view)
+
+
 def _stream_handle(stream=None) -> int:
     global _torch_c
     if stream is not None:
@@ -292,12 +312,12 @@ def append_fused(view: PoolView, kv_a, gamma, cos, sin, slot_mapping, eps: float
     latent_ptr, latent_stride = (0, 0) if latent_out is None else (latent_out.data_ptr(), latent_out.stride()[0])
     rope_ptr, rope_stride = (0, 0) if rope_out is None else (rope_out.data_ptr(), rope_out.stride()[0])
     cos_stride, sin_stride = cos.stride(), sin.stride()
-    a = _pack_producer(bytes(view), _ptr(kv_a), kv_a.stride()[0] if n else LATENT_DIM + ROPE_DIM, _ptr(gamma), eps,
+    a = _pack_producer(_view_bytes(view), _ptr(kv_a), kv_a.stride()[0] if n else LATENT_DIM + ROPE_DIM, _ptr(gamma), eps,
                      cos.data_ptr(), cos_stride[0] if len(cos_stride) == 2 else 0,
                      sin.data_ptr(), sin_stride[0] if len(sin_stride) == 2 else 0, slot_mapping.data_ptr(), n,
                      q_ptr, q_token_stride, q_head_stride, heads, latent_ptr, latent_stride, rope_ptr, rope_stride,
                      _ptr(rstd_out))
-    check(lib.b200kv_append_fused(a, _stream_handle(stream), _ptr(status)))
+    check(_append_fused(a, _stream_handle(stream), _ptr(status)))
 
 
 def mx_quant_e4m3(x, q, scales, stream=None) -> None:
@@ -334,7 +354,7 @@ def indexer_topk(q_fp8, q_scale, weights, key_pool, k_scale, block_table, kv_len
                     _ptr(k_scale), key_pool.shape[0], _ptr(block_table), block_table.shape[1], _ptr(kv_len),
                     batch, block_size, max_kv_len, k, index.data_ptr(), n_sel.data_ptr(), ws.data_ptr(), ws.numel(), variant,
                     _ptr(rows_out))
-    check(lib.b200kv_indexer_topk(a, _stream_handle(stream), _ptr(status)))
+    check(_indexer_topk(a, _stream_handle(stream), _ptr(status)))
     if scores_out is not None:
         stride = (max_kv_len + 3) & ~3  # the scores lie first in the workspace, [batch][stride] fp32
         scores_out.append(ws[: batch * stride * 4].view(torch.float32).view(batch, stride))
@@ -372,7 +392,7 @@ def mla_decode(q, view: PoolView, block_table, kv_len, block_size: int, scale: f
     quantisation written by the same launch."""
     args = _decode_args(q, view, block_table, kv_len, block_size, scale, out, lse, kv_begin, workspace, max_ctas, stable_tables,
                         partial, variant, new_rows, row_index, quantised)
-    check(lib.b200kv_mla_decode(args, _stream_handle(stream), _ptr(status)))
+    check(_mla_decode(args, _stream_handle(stream), _ptr(status)))
 
 
 def _decode_args(q, view: PoolView, block_table, kv_len, block_size: int, scale: float, out=None, lse=None, kv_begin=None,
@@ -392,7 +412,7 @@ def _decode_args(q, view: PoolView, block_table, kv_len, block_size: int, scale:
         rope, rope_stride = _ptr(new_rope), new_rope.stride()[0]
     rows, rows_stride = (0, 0) if row_index is None else (row_index.data_ptr(), row_index.stride()[0])
     fp8, scales = (0, 0) if quantised is None else (_ptr(quantised[0]), _ptr(quantised[1]))
-    return _pack_decode(_ptr(q), q_seq_stride, q_head_stride, bytes(view), table, max_blocks, _ptr(kv_len), _ptr(kv_begin),
+    return _pack_decode(_ptr(q), q_seq_stride, q_head_stride, _view_bytes(view), table, max_blocks, _ptr(kv_len), _ptr(kv_begin),
                       batch, heads, block_size, scale, _ptr(out), _ptr(lse), o, m, l, ws, ws_bytes, variant, max_ctas,
                       latent, latent_stride, rope, rope_stride, 1 if stable_tables else 0, rows, rows_stride, fp8, scales)
 
@@ -401,10 +421,8 @@ def mla_decode_static(q, view: PoolView, block_table, kv_len, block_size: int, s
                       kv_begin=None, partial=None, max_ctas: int = 0, status=None, stream=None) -> None:
     """b200kv_mla_decode_static: the same attention, with the library's built-in scratch instead of a
     workspace tensor; nothing is allocated on the device by the call."""
-    lib.b200kv_mla_decode_static.restype = c_int32
-    lib.b200kv_mla_decode_static.argtypes = [c_void_p, c_void_p, c_void_p]
     args = _decode_args(q, view, block_table, kv_len, block_size, scale, out, lse, kv_begin, None, max_ctas, False, partial)
-    check(lib.b200kv_mla_decode_static(args, _stream_handle(stream), _ptr(status)))
+    check(_mla_decode_static(args, _stream_handle(stream), _ptr(status)))
 
 
 def lse_merge(partial_o, partial_m, partial_l, out, lse=None, stream=None) -> None:

@@ -1,5 +1,6 @@
 """What the Python binding hands to the library: refusals come back as the library's, and calls that need no array take none.
 All of it answers on the host (a stream of handle 0 stands for the current one)."""
+import ctypes
 from types import SimpleNamespace
 
 import pytest
@@ -75,3 +76,24 @@ def test_further_dimensions_and_wrong_counts():
             _decode(partial=partial)
     with pytest.raises(ValueError):
         _decode(new_rows=(_aligned(2, 512), _aligned(2, 64), None))
+
+
+def test_argument_types_are_checked():
+    """The library's functions take a pointer to their own structure (or the structure), and calls a pool view: anything else
+    would be read as addresses."""
+    wrong = b200kv.KvCache()
+    for call in (_append_fused, _decode, lambda **k: _decode(b200kv.mla_decode_static, **k)):
+        with pytest.raises(TypeError):
+            call(view=wrong)
+        with pytest.raises(TypeError):
+            call(view=bytes(_view()))
+    for name, own, other in (("b200kv_mla_decode", b200kv.DecodeArgs, b200kv.IndexerArgs),
+                             ("b200kv_mla_decode_static", b200kv.DecodeArgs, b200kv.ProducerArgs),
+                             ("b200kv_append_fused", b200kv.ProducerArgs, b200kv.DecodeArgs),
+                             ("b200kv_indexer_topk", b200kv.IndexerArgs, b200kv.ProducerArgs)):
+        fn = getattr(b200kv.lib, name)
+        for args in (own(), ctypes.byref(own()), None):
+            assert fn(args, None, None) != b200kv.ERR_RUNTIME  # taken, and refused or found empty by the library
+        for args in (other(), ctypes.byref(other()), bytes(ctypes.sizeof(own)), 4096):
+            with pytest.raises(ctypes.ArgumentError):
+                fn(args, None, None)
