@@ -216,14 +216,16 @@ __global__ void __launch_bounds__(kLatentWords / 2)
   const float4* src = reinterpret_cast<const float4*>(part_o + row * B200KV_LATENT_DIM) + threadIdx.x;
   const int64_t step = rows * (B200KV_LATENT_DIM / 4);  // float4s from one part to the next
   float4 v[kAhead];
-  auto load = [&](int first) {
+  auto load = [&](int left) {  // the next kAhead parts of the `left` that have not been loaded
 #pragma unroll
     for (int k = 0; k < kAhead; ++k) {
-      if (first + k < n_parts) v[k] = src[(first + k) * step];
+      if (k < left) v[k] = *src;
+      src += step;
     }
   };
-  load(0);
+  load(n_parts);
   float m = -INFINITY, l = 0.0f, big = -INFINITY;  // (m, l) of part `lane` of the present 32
+#pragma unroll 1
   for (int r = lane; r < n_parts; r += 32) {
     const float lr = part_l[r * rows + row], mr = part_m[r * rows + row];
     if (r == lane) {
@@ -236,21 +238,26 @@ __global__ void __launch_bounds__(kLatentWords / 2)
   for (int off = 16; off > 0; off >>= 1) big = fmaxf(big, __shfl_xor_sync(0xffffffffu, big, off));
   float total = 0.0f;
   float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll 1
   for (int r0 = 0; r0 < n_parts; r0 += 32) {
     if (r0 > 0) {
       const int r = r0 + lane;
       l = r < n_parts ? part_l[r * rows + row] : 0.0f;
       m = r < n_parts ? part_m[r * rows + row] : -INFINITY;
     }
-    const float weight = l > 0.0f ? expf(m - big) : 0.0f;
-    total += weight > 0.0f ? l * weight : 0.0f;
+    // A part counts when it has l > 0, whatever its weight turns out to be: one with a NaN or an infinity in it makes the
+    // row NaN instead of being left out.
+    const unsigned live = __ballot_sync(0xffffffffu, l > 0.0f);
+    const float weight = expf(m - big);
+    total += l > 0.0f ? l * weight : 0.0f;
     const int here = n_parts - r0 < 32 ? n_parts - r0 : 32;
+#pragma unroll 1
     for (int k0 = 0; k0 < here; k0 += kAhead) {
-      if (r0 + k0 > 0) load(r0 + k0);
+      if (r0 + k0 > 0) load(n_parts - r0 - k0);
 #pragma unroll
       for (int k = 0; k < kAhead; ++k) {
         const float w = __shfl_sync(0xffffffffu, weight, (k0 + k) & 31);
-        if (k0 + k < here && w > 0.0f) {  // (an empty part's data may be anything)
+        if ((live >> (k0 + k)) & 1u) {  // (an empty part's data may be anything)
           acc.x = fmaf(v[k].x, w, acc.x);
           acc.y = fmaf(v[k].y, w, acc.y);
           acc.z = fmaf(v[k].z, w, acc.z);

@@ -148,6 +148,46 @@ def test_kv_range_shards_merge_to_whole(variant):
     assert np.abs(lse.cpu().numpy() - want_lse).max() <= 1e-4
 
 
+@pytest.mark.parametrize("parts,odd", [(1, 0), (2, 1), (3, 0), (9, 8), (40, 33)])
+@pytest.mark.parametrize("rows", [6, 8192])
+def test_merge_leaves_no_part_out_that_has_a_sum(parts, odd, rows):
+    """A part counts when its l is above zero: one whose m or data is not finite makes its row NaN, and is not dropped
+    without a trace. A part with l = 0 (or NaN) is empty and its data may be anything. Six kinds of rows, in turn."""
+    g = torch.Generator(device="cuda")
+    g.manual_seed(parts)
+    o = torch.randn((parts, rows, 512), generator=g, device="cuda")
+    m = torch.rand((parts, rows), generator=g, device="cuda")
+    l = torch.rand((parts, rows), generator=g, device="cuda") + 0.5
+    nan, inf = float("nan"), float("inf")
+    m[odd, 0::6] = nan
+    m[odd, 1::6] = inf
+    m[:, 2::6] = -inf
+    l[odd, 3::6], o[odd, 3::6], m[odd, 3::6] = 0.0, nan, nan
+    l[odd, 4::6], o[odd, 4::6] = nan, nan
+    o[odd, 5::6] = nan
+    if parts > 1:
+        m[odd, 5::6] = -200.0  # a weight of zero beside the others
+    out = torch.zeros((rows, 512), dtype=torch.bfloat16, device="cuda")
+    lse = torch.zeros(rows, device="cuda")
+    b200kv.lse_merge(o, m, l, out, lse)
+    for kind in (0, 1, 2, 5):
+        assert out[kind::6].isnan().all(), kind
+    rest = [p for p in range(parts) if p != odd]
+    for kind in (3, 4):
+        got, got_lse = out[kind::6].double(), lse[kind::6].double()
+        if not rest:
+            assert (got == 0).all() and (got_lse == -inf).all()
+            continue
+        mm, ll = m[rest, kind::6].double(), l[rest, kind::6].double()
+        big = mm.amax(0)
+        w = (mm - big).exp()
+        total = (ll * w).sum(0)
+        want = (o[rest, kind::6].double() * w[..., None]).sum(0) / total[:, None]
+        # bf16 output, and at most 40 fp32 additions of terms below 5
+        assert ((got - want).abs() <= 2.0**-8 * want.abs() + 40 * 5 * 2.0**-24).all()
+        assert (got_lse - (big + total.log())).abs().max() <= 1e-5
+
+
 def test_simt_handles_other_head_counts():
     bs, blocks = 64, 8
     kv_len = np.array([150, 64], dtype=np.int32)
