@@ -199,27 +199,38 @@ __global__ void __launch_bounds__(kThreads, 1) MlaDecodeSimtKernel(SimtParams p)
   }
 }
 
-// One CTA per (sequence, head) row: merges n_parts partials laid out [part][rows]. A thread owns four columns and has eight
-// parts' data in flight, the first eight before the weights are known; every warp works the weights out for itself, a lane
-// a part. Bound by two trips to memory: a warp per row, which walked the parts one after the other (twice, the maxima
-// first), and no overlap with the kernel before it took 7.0 us for 64 rows of eight parts behind a decode call, this 3.1.
+// Merges n_parts partials laid out [part][rows], a row being a (sequence, head). A thread has eight float4s of 512 columns x
+// parts in flight, the first before the weights are known; every warp works the weights out for itself, a lane a part.
+// kPerThread float4s of a row to a thread, so 128 / kPerThread threads to a row. Bound by two trips to memory while the rows
+// are few, so a row gets a CTA (kPerThread 1: 64 rows of eight parts behind a decode call 3.1 us; a warp per row that walked
+// the parts one after the other, twice, and no overlap with the kernel before it: 7.0 us); by HBM once they are many, where
+// a CTA's life is too short for what it loads and a row gets a warp (LaunchLseMerge has the line and both sides' times).
 // emit_partial != 0 writes the un-normalised merged (m, l, O) instead of (out, lse).
-__global__ void __launch_bounds__(kLatentWords / 2)
+constexpr int kMergeThreads = 128;
+
+template <int kPerThread>
+__global__ void __launch_bounds__(kMergeThreads)
     LseMergeKernel(const float* __restrict__ part_o, const float* __restrict__ part_m,
                    const float* __restrict__ part_l, int32_t n_parts, int64_t rows, __nv_bfloat16* out, float* lse,
                    float* merged_o, float* merged_m, float* merged_l, int32_t emit_partial) {
-  constexpr int kAhead = 8;
+  constexpr int kAhead = 8 / kPerThread;
+  constexpr int kRowThreads = B200KV_LATENT_DIM / 4 / kPerThread;
   GridDependencyTrigger();
   GridDependencyWait();
   const int lane = threadIdx.x & 31;
-  const int64_t row = blockIdx.x;
-  const float4* src = reinterpret_cast<const float4*>(part_o + row * B200KV_LATENT_DIM) + threadIdx.x;
+  const int at = threadIdx.x % kRowThreads;  // this thread's float4s of the row: at, at + kRowThreads, ...
+  const int64_t row = static_cast<int64_t>(blockIdx.x) * (kMergeThreads / kRowThreads) + threadIdx.x / kRowThreads;
+  if (row >= rows) return;  // (whole warps)
+  const float4* src = reinterpret_cast<const float4*>(part_o + row * B200KV_LATENT_DIM) + at;
   const int64_t step = rows * (B200KV_LATENT_DIM / 4);  // float4s from one part to the next
-  float4 v[kAhead];
+  float4 v[kAhead][kPerThread];
   auto load = [&](int left) {  // the next kAhead parts of the `left` that have not been loaded
 #pragma unroll
     for (int k = 0; k < kAhead; ++k) {
-      if (k < left) v[k] = *src;
+      if (k < left) {
+#pragma unroll
+        for (int c = 0; c < kPerThread; ++c) v[k][c] = src[c * kRowThreads];
+      }
       src += step;
     }
   };
@@ -237,7 +248,9 @@ __global__ void __launch_bounds__(kLatentWords / 2)
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) big = fmaxf(big, __shfl_xor_sync(0xffffffffu, big, off));
   float total = 0.0f;
-  float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  float4 acc[kPerThread];
+#pragma unroll
+  for (int c = 0; c < kPerThread; ++c) acc[c] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll 1
   for (int r0 = 0; r0 < n_parts; r0 += 32) {
     if (r0 > 0) {
@@ -258,10 +271,13 @@ __global__ void __launch_bounds__(kLatentWords / 2)
       for (int k = 0; k < kAhead; ++k) {
         const float w = __shfl_sync(0xffffffffu, weight, (k0 + k) & 31);
         if ((live >> (k0 + k)) & 1u) {  // (an empty part's data may be anything)
-          acc.x = fmaf(v[k].x, w, acc.x);
-          acc.y = fmaf(v[k].y, w, acc.y);
-          acc.z = fmaf(v[k].z, w, acc.z);
-          acc.w = fmaf(v[k].w, w, acc.w);
+#pragma unroll
+          for (int c = 0; c < kPerThread; ++c) {
+            acc[c].x = fmaf(v[k][c].x, w, acc[c].x);
+            acc[c].y = fmaf(v[k][c].y, w, acc[c].y);
+            acc[c].z = fmaf(v[k][c].z, w, acc[c].z);
+            acc[c].w = fmaf(v[k][c].w, w, acc[c].w);
+          }
         }
       }
     }
@@ -269,21 +285,25 @@ __global__ void __launch_bounds__(kLatentWords / 2)
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) total += __shfl_xor_sync(0xffffffffu, total, off);
   if (emit_partial) {
-    reinterpret_cast<float4*>(merged_o + row * B200KV_LATENT_DIM)[threadIdx.x] = acc;
-    if (threadIdx.x == 0) {
+#pragma unroll
+    for (int c = 0; c < kPerThread; ++c) reinterpret_cast<float4*>(merged_o + row * B200KV_LATENT_DIM)[at + c * kRowThreads] = acc[c];
+    if (at == 0) {
       merged_m[row] = big;
       merged_l[row] = total;
     }
     return;
   }
   const float inv = total > 0.0f ? 1.0f / total : 0.0f;
-  const __nv_bfloat162 lo = __floats2bfloat162_rn(acc.x * inv, acc.y * inv);
-  const __nv_bfloat162 hi = __floats2bfloat162_rn(acc.z * inv, acc.w * inv);
-  uint2 packed;
-  packed.x = *reinterpret_cast<const uint32_t*>(&lo);
-  packed.y = *reinterpret_cast<const uint32_t*>(&hi);
-  reinterpret_cast<uint2*>(out + row * B200KV_LATENT_DIM)[threadIdx.x] = packed;
-  if (threadIdx.x == 0 && lse) lse[row] = total > 0.0f ? big + logf(total) : -INFINITY;
+#pragma unroll
+  for (int c = 0; c < kPerThread; ++c) {
+    const __nv_bfloat162 lo = __floats2bfloat162_rn(acc[c].x * inv, acc[c].y * inv);
+    const __nv_bfloat162 hi = __floats2bfloat162_rn(acc[c].z * inv, acc[c].w * inv);
+    uint2 packed;
+    packed.x = *reinterpret_cast<const uint32_t*>(&lo);
+    packed.y = *reinterpret_cast<const uint32_t*>(&hi);
+    reinterpret_cast<uint2*>(out + row * B200KV_LATENT_DIM)[at + c * kRowThreads] = packed;
+  }
+  if (at == 0 && lse) lse[row] = total > 0.0f ? big + logf(total) : -INFINITY;
 }
 
 }  // namespace
@@ -302,9 +322,14 @@ size_t SimtWorkspaceBytes(int32_t batch, int32_t heads, int32_t sms) {
 
 int32_t LaunchLseMerge(const float* part_o, const float* part_m, const float* part_l, int32_t n_parts, int64_t rows,
                        void* out, float* lse, float* merged_o, float* merged_m, float* merged_l, cudaStream_t stream) {
-  return CheckCuda(LaunchOverlapped(LseMergeKernel, dim3(static_cast<unsigned>(rows)), dim3(kLatentWords / 2), 0, stream, part_o,
-                                    part_m, part_l, n_parts, rows, static_cast<__nv_bfloat16*>(out), lse, merged_o, merged_m,
-                                    merged_l, merged_o != nullptr ? 1 : 0),
+  // us with a CTA and with a warp a row: 2 parts of 1,024 / 2,048 / 4,096 / 8,192 rows 2.43 / 3.82 / 5.89 / 10.1 and
+  // 2.25 / 2.78 / 3.07 / 4.59; 2,048 rows of 6 / 8 parts 4.24 / 4.41 and 4.17 / 5.01; 4,096 rows of 8 / 12 / 16 parts
+  // 7.13 / 15.5 / 21.8 and 6.10 / 14.3 / 22.0. With more parts and more rows both are at the roof.
+  const bool warp_a_row = rows >= 2048 && n_parts <= (rows >= 4096 ? 12 : 6);
+  const int64_t ctas = warp_a_row ? (rows + 3) / 4 : rows;
+  return CheckCuda(LaunchOverlapped(warp_a_row ? LseMergeKernel<4> : LseMergeKernel<1>, dim3(static_cast<unsigned>(ctas)),
+                                    dim3(kMergeThreads), 0, stream, part_o, part_m, part_l, n_parts, rows,
+                                    static_cast<__nv_bfloat16*>(out), lse, merged_o, merged_m, merged_l, merged_o != nullptr ? 1 : 0),
                    "lse merge launch");
 }
 

@@ -148,8 +148,8 @@ def test_kv_range_shards_merge_to_whole(variant):
     assert np.abs(lse.cpu().numpy() - want_lse).max() <= 1e-4
 
 
-@pytest.mark.parametrize("parts,odd", [(1, 0), (2, 1), (3, 0), (9, 8), (40, 33)])
-@pytest.mark.parametrize("rows", [6, 8192])
+@pytest.mark.parametrize("parts,odd", [(1, 0), (2, 1), (3, 0), (6, 2), (7, 6), (9, 8), (12, 5), (13, 12), (40, 33)])
+@pytest.mark.parametrize("rows", [6, 2047, 2049, 4096, 8192])
 def test_merge_leaves_no_part_out_that_has_a_sum(parts, odd, rows):
     """A part counts when its l is above zero: one whose m or data is not finite makes its row NaN, and is not dropped
     without a trace. A part with l = 0 (or NaN) is empty and its data may be anything. Six kinds of rows, in turn."""
