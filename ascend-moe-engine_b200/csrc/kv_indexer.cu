@@ -153,7 +153,15 @@ constexpr int kListKeys = 4096;  // keys that can be collected
 constexpr int kMaxCluster = 16;
 constexpr int kTokensPerCta = 4096;
 constexpr int kFewTokens = 128;  // up to so many keys are ordered by comparing all with all (7.2 us a call; with 500 keys 17.5 against 8.9)
-constexpr uint32_t kMostComparisons = 400000;  // per CTA, some 6 us of it: what sorting the list takes
+// Comparisons, per CTA and key of the padded list, from which on sorting the list is the shorter way: a CTA compares some
+// 20,000 pairs a us. (512 keys in groups of 64 / 128 / 256 equal scores, one CTA: 1.6 / 3.2 / 6.0 us compared.)
+constexpr uint32_t kComparisonsPerKey = 100;
+// What SortKeys makes of a list of so many keys: a power of two, four keys to each thread of a warp at least.
+__host__ __device__ constexpr uint32_t PaddedKeys(uint32_t keys) {
+  uint32_t padded = 128;
+  while (padded < keys) padded <<= 1;
+  return padded;
+}
 
 struct SelectParams {
   const float* scores;
@@ -172,8 +180,8 @@ struct SelectParams {
 };
 
 struct SelectShared {
-  uint64_t all[kListKeys];      // the list: the keys up to the bound, bin after bin; filled where this CTA's entries' bins lie
-  uint64_t scratch[kListKeys];  // this CTA's keys on their way to the lists; the sort's other buffer
+  alignas(16) uint64_t all[kListKeys];      // the list: the keys up to the bound, bin after bin; filled where this CTA's entries' bins lie
+  alignas(16) uint64_t scratch[kListKeys];  // this CTA's keys on their way to the lists; the sort's other buffer
   uint16_t place[kListKeys];    // ... and where they go
   alignas(16) uint32_t hist[2][kBins];  // by parity of the pass: the peers read one while the next is cleared
   alignas(16) uint32_t peers[kMaxCluster][kBins];
@@ -186,57 +194,64 @@ struct SelectShared {
   uint32_t chosen[3];  // bin, keys in the bins before it, keys in it
 };
 
-// Bitonic sort, ascending, of kEach * threads keys (a power of two; threads <= 1024, a multiple of 32, the block's first
-// ones): keys tid + j * threads of `data` in register j. Partners `threads` or more away sit in the same thread, less than
-// 32 away in the same warp; the others are exchanged through the two buffers in turn, one barrier a step.
-template <int kEach>
+// Bitonic sort, ascending, of 4 * threads keys (threads a power of two, 32 .. 1024; the block's first ones): thread t has
+// keys 4 t .. 4 t + 3 in registers. Partners one or two away sit in the same thread, up to 64 away in the same warp; the
+// others are exchanged through the two buffers in turn, one barrier a step. A step costs its latencies and, above all, its
+// branches, so it has none: 512 / 1,024 / 2,048 keys take 2.3 / 4.2 / 7.2 us (branches on the two sides of an exchange: 6 /
+// 11 / 24 us).
 __device__ void SortKeys(uint64_t* data, uint64_t* other, int threads) {
   const int tid = threadIdx.x;
-  const int total = kEach * threads;
-  uint64_t key[kEach];
+  uint64_t key[4];
+  auto read = [&](const uint64_t* from, int thread, uint64_t (&to)[4]) {
+    const ulonglong2 a = reinterpret_cast<const ulonglong2*>(from)[2 * thread], b = reinterpret_cast<const ulonglong2*>(from)[2 * thread + 1];
+    to[0] = a.x, to[1] = a.y, to[2] = b.x, to[3] = b.y;
+  };
+  auto write = [&](uint64_t* to) {
+    reinterpret_cast<ulonglong2*>(to)[2 * tid] = make_ulonglong2(key[0], key[1]);
+    reinterpret_cast<ulonglong2*>(to)[2 * tid + 1] = make_ulonglong2(key[2], key[3]);
+  };
+  auto order_pair = [&](uint64_t& a, uint64_t& b, bool up) {  // a before b, or the other way round
+    const uint64_t x = a, y = b;
+    const bool swap = (x > y) == up;
+    a = swap ? y : x;
+    b = swap ? x : y;
+  };
+  auto meet = [&](const uint64_t (&theirs)[4], bool smaller) {
 #pragma unroll
-  for (int j = 0; j < kEach; ++j) key[j] = data[tid + j * threads];
-  asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory");
-  uint64_t* buffer = data;
-  for (int size = 2; size <= total; size <<= 1) {
-    for (int stride = size >> 1; stride > 0; stride >>= 1) {
-      if (stride >= threads) {
-        if constexpr (kEach > 1) {
-          const int apart = stride / threads;  // 1 or 2
-#pragma unroll
-          for (int j = 0; j < kEach; ++j) {
-#pragma unroll
-            for (int a = 1; a < kEach; a <<= 1) {
-              if (a == apart && (j & a) == 0) {
-                const bool ascending = ((tid + j * threads) & size) == 0;
-                const uint64_t x = key[j], y = key[j | a];
-                const bool swap = (x > y) == ascending;
-                key[j] = swap ? y : x;
-                key[j | a] = swap ? x : y;
-              }
-            }
-          }
-        }
-        continue;
-      }
-      if (stride >= 32) {
-#pragma unroll
-        for (int j = 0; j < kEach; ++j) buffer[tid + j * threads] = key[j];
-        asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory");
-      }
-#pragma unroll
-      for (int j = 0; j < kEach; ++j) {
-        const int e = tid + j * threads;
-        const uint64_t theirs = stride >= 32 ? buffer[e ^ stride] : __shfl_xor_sync(0xffffffffu, key[j], stride);
-        const bool keep_smaller = ((e & stride) == 0) == ((e & size) == 0);
-        if (keep_smaller ? theirs < key[j] : theirs > key[j]) key[j] = theirs;
-      }
-      if (stride >= 32) buffer = buffer == data ? other : data;
+    for (int j = 0; j < 4; ++j) {
+      const bool take = (theirs[j] < key[j]) == smaller;  // (no branches: they diverge)
+      key[j] = take ? theirs[j] : key[j];
     }
+  };
+  read(data, tid, key);
+  asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory");
+  order_pair(key[0], key[1], true);
+  order_pair(key[2], key[3], false);
+  uint64_t* buffer = data;
+  for (int size = 1; size <= threads; size <<= 1) {  // in threads: runs of 4 * size keys
+    const bool up = (tid & size) == 0;
+    int stride = size >> 1;  // in threads
+    for (; stride >= 32; stride >>= 1) {
+      write(buffer);
+      asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory");
+      uint64_t theirs[4];
+      read(buffer, tid ^ stride, theirs);
+      meet(theirs, ((tid & stride) == 0) == up);
+      buffer = buffer == data ? other : data;
+    }
+    for (; stride > 0; stride >>= 1) {
+      uint64_t theirs[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) theirs[j] = __shfl_xor_sync(0xffffffffu, key[j], stride);
+      meet(theirs, ((tid & stride) == 0) == up);
+    }
+    order_pair(key[0], key[2], up);
+    order_pair(key[1], key[3], up);
+    order_pair(key[0], key[1], up);
+    order_pair(key[2], key[3], up);
   }
   asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory");
-#pragma unroll
-  for (int j = 0; j < kEach; ++j) data[tid + j * threads] = key[j];
+  write(data);
 }
 
 __global__ void __launch_bounds__(kSortThreads) IndexerSelectKernel(SelectParams p) {
@@ -371,6 +386,10 @@ __global__ void __launch_bounds__(kSortThreads) IndexerSelectKernel(SelectParams
   cluster_sync();
   img_lo = __reduce_min_sync(0xffffffffu, sh.lo[lane & (cluster - 1)]);
   img_hi = __reduce_max_sync(0xffffffffu, sh.hi[lane & (cluster - 1)]);
+  if (img_lo == img_hi) {  // all scores equal: the first positions, in order
+    for (int i = rank * kSortThreads + tid; i < kept; i += kSortThreads << cluster_log2) write(static_cast<uint64_t>(i), i);
+    return;
+  }
 
   // The wanted key is the `rank_left`-th of those with a value in [lo, hi]; all `taken` keys below are wanted, `run` of
   // them those of CTA number `warp`. The value is the image or, when there are too many keys of one image, the position
@@ -454,8 +473,8 @@ __global__ void __launch_bounds__(kSortThreads) IndexerSelectKernel(SelectParams
     if (total <= enough) {  // (a bin of one position holds one key: the passes end)
       uint32_t squares = taken * taken;
       for (int w = 0; w < kBins / 32; ++w) squares += sh.warp_b[w];
-      dense = squares > (kMostComparisons << cluster_log2);
-      break;
+      dense = squares > (kComparisonsPerKey * PaddedKeys(total)) << cluster_log2;
+      if (!dense || total <= kMaxK) break;  // (a pass more, 2.5 us, is shorter than sorting 4,096 keys instead of 2,048)
     }
     if (warp < cluster) {
       uint32_t sum = 0;
@@ -518,20 +537,10 @@ __global__ void __launch_bounds__(kSortThreads) IndexerSelectKernel(SelectParams
     return;
   }
   if (rank != 0) return;
-  int padded = 32;
-  while (padded < keys) padded <<= 1;
+  const int padded = static_cast<int>(PaddedKeys(total));
   for (int i = keys + tid; i < padded; i += kSortThreads) sh.all[i] = ~0ull;
   __syncthreads();
-  const int threads = min(padded, kSortThreads);
-  if (tid < threads) {
-    if (padded <= kSortThreads) {
-      SortKeys<1>(sh.all, sh.scratch, threads);
-    } else if (padded == 2 * kSortThreads) {
-      SortKeys<2>(sh.all, sh.scratch, threads);
-    } else {
-      SortKeys<4>(sh.all, sh.scratch, threads);
-    }
-  }
+  if (tid < padded / 4) SortKeys(sh.all, sh.scratch, padded / 4);
   __syncthreads();
   for (int i = tid; i < kept; i += kSortThreads) write(sh.all[i], i);
 }

@@ -261,6 +261,30 @@ def test_indexer_selection_matches_oracle_bit_for_bit(lens, k):
     assert np.array_equal(index.cpu().numpy(), exp_index), "selection differs from the oracle"
 
 
+@pytest.mark.parametrize("length,k", [(200, 64), (200, 256), (400, 300), (600, 512), (900, 1024), (1100, 700), (2048, 2048), (3000, 1024),
+                                      (3000, 2048), (4096, 2048), (9000, 1500), (40000, 2048)])
+@pytest.mark.parametrize("values", [1, 2, 4, 8, 32])
+def test_indexer_selection_of_tied_scores(length, k, values):
+    """Scores that take few values: ties go by position. Lists on both sides of the line between comparing and sorting, every
+    padded length of the sort, and lists that take a pass more before they are sorted."""
+    bs = 64
+    blocks = (length + bs - 1) // bs
+    q = torch.zeros((1, 1, 128), dtype=torch.uint8, device="cuda")
+    q[..., 0] = 0x38  # 1.0
+    key = torch.zeros((blocks * bs, 128), dtype=torch.uint8, device="cuda")
+    key[:, 0] = 0x38
+    g = torch.Generator(device="cuda")
+    g.manual_seed(length + values)
+    ks = torch.randint(0, values, (blocks * bs,), generator=g, device="cuda").float() + 1.0
+    ones = torch.ones((1, 1), device="cuda")
+    index, n_sel = b200kv.indexer_topk(q, ones, ones.bfloat16(), key, ks, torch.arange(blocks, device="cuda", dtype=torch.int32).view(1, -1),
+                                       torch.tensor([length], device="cuda", dtype=torch.int32), bs, length, k, variant=b200kv.INDEXER_EXACT)
+    kept = min(length, k)
+    assert n_sel.item() == kept
+    want = torch.sort(ks[:length], descending=True, stable=True)[1][:kept].int()
+    assert torch.equal(index[0, :kept], want) and (index[0, kept:] == -1).all()
+
+
 def test_indexer_selection_of_more_sequences_than_a_grid_is_high():
     """65,600 sequences of one to three tokens: the batch exceeds what a grid's second and third extents can hold."""
     B, bs, k = 65600, 64, 2
