@@ -783,7 +783,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       p.user_m[at] = m_nat;
       p.user_l[at] = total;
     } else if (p.lse != nullptr) {
-      p.lse[at] = total > 0.0f ? m_nat + logf(total) : -INFINITY;
+      p.lse[at] = total == 0.0f ? -INFINITY : m_nat + logf(total);
     }
   };
   // (m, l) of this CTA's token range: lane j < 16 of a softmax warp takes row j of the warp's sixteen.
@@ -805,7 +805,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     // Nobody to exchange with: out of the accumulators straight into the rows.
     float* s_norm = reinterpret_cast<float*>(smem + kOffW);
     if (has_row) {
-      s_norm[h_row] = l_row > 0.0f ? 1.0f / l_row : 0.0f;
+      s_norm[h_row] = l_row == 0.0f ? 0.0f : 1.0f / l_row;
       emit_ml(h_row, m_row, l_row);
     }
     __syncthreads();
@@ -936,14 +936,14 @@ __global__ void __launch_bounds__(kThreads, 1)
       for (int off = 4; off < 32; off <<= 1) big = fmaxf(big, __shfl_xor_sync(0xffffffffu, big, off));
 #pragma unroll
       for (int k = 0; k < 2; ++k) {
-        m[k] = l[k] > 0.0f ? exp2f(m[k] - big) : 0.0f;  // the range's weight
+        m[k] = l[k] > 0.0f ? exp2f(m[k] - big) : l[k];  // the range's weight: zero without a sum, NaN if that is NaN
         zero |= (lane >> 2) + 8 * k < share.ranges && !(m[k] > 0.0f);
         total = fmaf(l[k], m[k], total);
       }
 #pragma unroll
       for (int off = 4; off < 32; off <<= 1) total += __shfl_xor_sync(0xffffffffu, total, off);
       whole = !__any_sync(0xffffffffu, zero);  // (and: the previous quad's weights have been read)
-      const float norm = want_partial ? 1.0f : (total > 0.0f ? 1.0f / total : 0.0f);
+      const float norm = want_partial ? 1.0f : (total == 0.0f ? 0.0f : 1.0f / total);
 #pragma unroll
       for (int k = 0; k < 2; ++k) {
         const int s = (lane >> 2) + 8 * k;

@@ -157,3 +157,65 @@ def test_merge_of_many_parts_in_every_shape(batch, quantised):
             assert torch.equal(codes[0].view(batch, -1), fp8) and torch.equal(codes[1].view(batch, -1), scales)
     assert ((got[0][0] - got[1][0]).abs() <= 2e-3 + 1e-2 * got[1][0].abs().amax(dim=2, keepdim=True)).all()
     assert ((got[0][1] - got[1][1]).abs() <= 1e-4).all()
+
+
+def _decode_dev(q, pool, table, kv_len, bs, variant=b200kv.DECODE_AUTO, partial=False, max_ctas=0):
+    """The call on torch tensors: (out, lse), or (o, m, l) of a partial."""
+    batch, heads = q.shape[:2]
+    ws = torch.empty(b200kv.decode_workspace_bytes(batch, heads, max_ctas), dtype=torch.uint8, device="cuda")
+    status = b200kv.new_status()
+    if partial:
+        got = (torch.zeros((batch, heads, 512), device="cuda"), torch.zeros((batch, heads), device="cuda"), torch.zeros((batch, heads), device="cuda"))
+        kw = {"partial": got}
+    else:
+        got = (torch.zeros((batch, heads, 512), dtype=torch.bfloat16, device="cuda"), torch.zeros((batch, heads), device="cuda"))
+        kw = {"out": got[0], "lse": got[1]}
+    b200kv.mla_decode(q, b200kv.pool_view(pool), table, kv_len, bs, 1.0 / 24.0, workspace=ws, status=status, variant=variant,
+                      max_ctas=max_ctas, **kw)
+    status_ok(status)
+    return got
+
+
+def _case(kv_len, bs, heads=64, seed=3):
+    kv_len = np.array(kv_len, dtype=np.int32)
+    blocks = int(sum(scenarios.blocks_for(int(n), bs) for n in kv_len)) + 3
+    table = scenarios.build_tables(kv_len, bs, blocks, order=kvo.permutation(blocks))
+    g = torch.Generator(device="cuda")
+    g.manual_seed(seed)
+    pool = torch.randn((blocks * bs, 576), generator=g, device="cuda").bfloat16()
+    q = torch.randn((len(kv_len), heads, 576), generator=g, device="cuda").bfloat16()
+    rows = [torch.from_numpy(table[b, np.arange(n) // bs].astype(np.int64) * bs + np.arange(n) % bs).cuda() for b, n in enumerate(kv_len)]
+    return q, pool, to_dev_i32(table), to_dev_i32(kv_len), rows
+
+
+def _attention_f64(q, pool, rows):
+    out, lse = [], []
+    for b, r in enumerate(rows):
+        kv = pool[r].double()
+        s = q[b].double() @ kv.T / 24.0
+        lse.append(torch.logsumexp(s, dim=1))
+        out.append(torch.softmax(s, dim=1) @ kv[:, :512])
+    return torch.stack(out), torch.stack(lse)
+
+
+# (lengths, block size, heads): clusters of 16, of one and several head groups, of 8 and of 4, single CTAs, other geometries
+NOT_FINITE = [([700], 64, 64), ([2048], 64, 64), ([100, 64, 513], 64, 64), ([300] * 20, 64, 64), ([500] * 140, 64, 64),
+              ([700, 65], 16, 64), ([333], 1, 16), ([400] * 150, 64, 16)]
+
+
+@pytest.mark.parametrize("kv_len,bs,heads", NOT_FINITE)
+@pytest.mark.parametrize("at", ["first", "last"])
+def test_a_nan_in_a_sequence_makes_its_rows_nan(kv_len, bs, heads, at):
+    """However many CTAs share the sequence out; the other sequences are what they were. (The NaN sits in the rotary part of
+    one token's key, so it reaches a row through that token's weight only.)"""
+    q, pool, table, lens, rows = _case(kv_len, bs, heads)
+    clean, clean_lse = _decode_dev(q, pool, table, lens, bs)
+    hit = len(kv_len) // 2
+    pool[rows[hit][0 if at == "first" else -1], 575] = float("nan")
+    out, lse = _decode_dev(q, pool, table, lens, bs)
+    assert out[hit].isnan().all() and lse[hit].isnan().all()
+    rest = torch.arange(len(kv_len), device="cuda") != hit
+    assert torch.equal(out[rest], clean[rest]) and torch.equal(lse[rest], clean_lse[rest])
+    if heads == 64 and bs % 64 == 0:
+        _, _, l = _decode_dev(q, pool, table, lens, bs, partial=True)
+        assert l[hit].isnan().all() and l[rest].isfinite().all()
