@@ -219,3 +219,22 @@ def test_a_nan_in_a_sequence_makes_its_rows_nan(kv_len, bs, heads, at):
     if heads == 64 and bs % 64 == 0:
         _, _, l = _decode_dev(q, pool, table, lens, bs, partial=True)
         assert l[hit].isnan().all() and l[rest].isfinite().all()
+
+
+@pytest.mark.parametrize("kv_len,bs,heads", NOT_FINITE)
+def test_scores_of_minus_infinity_have_no_weight(kv_len, bs, heads):
+    """Tokens whose scores are all -infinity at the beginning of a sequence, past the first tile, count for nothing; a
+    sequence of nothing else is empty. (An infinity in the rotary part of the keys against a negative query.)"""
+    q, pool, table, lens, rows = _case(kv_len, bs, heads)
+    q[:, :, 575] = -1.0
+    dead = [min(len(r) - 1, 130) for r in rows]
+    for r, n in zip(rows, dead):
+        pool[r[:n], 575] = float("inf")
+    want, want_lse = _attention_f64(q, pool, [r[n:] for r, n in zip(rows, dead)])
+    out, lse = _decode_dev(q, pool, table, lens, bs)
+    assert ((out.double() - want).abs() <= 2e-3 + 1e-2 * want.abs().amax(dim=2, keepdim=True)).all()
+    assert (lse.double() - want_lse).abs().max() <= 1e-4
+    hit = len(kv_len) // 2
+    pool[rows[hit], 575] = float("inf")
+    out, lse = _decode_dev(q, pool, table, lens, bs)
+    assert (out[hit] == 0).all() and (lse[hit] == float("-inf")).all()
