@@ -812,7 +812,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         const int stage = g % kStages;
         const int tok0 = (t_lo + i) * kTile;
         const int valid = min(kTile, seq_len - tok0);
-        ok = __all_sync(0xffffffffu, BoundedWait(bar(&misc->s_full[buf]), (g >> 1) & 1, misc, p.status, 30));
+        ok = BoundedWait(bar(&misc->s_full[buf]), (g >> 1) & 1, misc, p.status, 30);  // (a lane's verdict; the barrier's vote joins them)
         ptx::TcFenceAfterSync();
         static_assert(kTile == 64, "one 16x256b.x8 load covers the 64 columns of a tile");
         uint32_t sr[32];
@@ -893,9 +893,9 @@ __global__ void __launch_bounds__(kThreads, 1)
           // comes here only to give up: there is no tile before it to wait for.)
           const int gp = g - 1;
           if (ok && i > 0) {
-            ok = __all_sync(0xffffffffu,
-                            BoundedWait(bar(&misc->kv_empty[gp % kStages][kGroups - 1]), (gp / kStages) & 1, misc, p.status, 31));
+            ok = BoundedWait(bar(&misc->kv_empty[gp % kStages][kGroups - 1]), (gp / kStages) & 1, misc, p.status, 31);
           }
+          __syncwarp();
           if (ptx::NamedBarrierOr(2, kSoftmaxThreads, !ok)) {
             ok = false;
             break;
@@ -951,7 +951,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       if (!ok) break;
 
       // ---- epilogue of the segment ----
-      ok = __all_sync(0xffffffffu, BoundedWait(bar(&misc->o_full), seg & 1, misc, p.status, 32));
+      ok = BoundedWait(bar(&misc->o_full), seg & 1, misc, p.status, 32);
       ptx::TcFenceAfterSync();
       const bool whole = (t_lo == 0 && t_hi == seq_tiles);
       const bool to_ws = !whole || p.force_ws != 0;
