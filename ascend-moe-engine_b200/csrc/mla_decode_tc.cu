@@ -964,7 +964,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       const float l_row = (lane & 8) ? l_hi : l_lo;
       const float m_nat = ((lane & 8) ? m_hi : m_lo) * 0.6931471805599453f;
       if (row_ok) {
-        misc->inv_l[head] = l_row > 0.0f ? 1.0f / l_row : 0.0f;
+        misc->inv_l[head] = l_row == 0.0f ? 0.0f : 1.0f / l_row;
         if (to_ws) {
           p.ws_m[slot * kHeads + head] = m_nat;
           p.ws_l[slot * kHeads + head] = l_row;
@@ -1246,7 +1246,8 @@ __global__ void __launch_bounds__(kGroups == 1 ? 128 : 256, kResident)
       float gsum = 0.0f;
 #pragma unroll
       for (int r = 0; r < kRounds; ++r) {
-        const float w = (l_mine[r] > 0.0f && new_big != -INFINITY) ? expf(m_mine[r] - new_big) : 0.0f;
+        // (a part without a sum has no weight, one whose sum is NaN a NaN)
+        const float w = (l_mine[r] > 0.0f && new_big != -INFINITY) ? expf(m_mine[r] - new_big) : l_mine[r] != l_mine[r] ? l_mine[r] : 0.0f;
         s_w[part_at(warp, 8 * r + (lane >> 2))][i] = w;
         gsum = fmaf(l_mine[r], w, gsum);
       }
@@ -1414,7 +1415,7 @@ __global__ void __launch_bounds__(kGroups == 1 ? 128 : 256, kResident)
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const float sum = s_sum[i];
-    const float inv = sum > 0.0f ? 1.0f / sum : 0.0f;
+    const float inv = sum == 0.0f ? 0.0f : 1.0f / sum;
 #pragma unroll
     for (int q = 0; q < kPasses; ++q) {
       const int64_t at = (row0 + i) * kLatent + dv_first + kGroupThreads * q;
@@ -1433,7 +1434,7 @@ __global__ void __launch_bounds__(kGroups == 1 ? 128 : 256, kResident)
       p.user_m[row0 + tid] = s_big[tid];
       p.user_l[row0 + tid] = sum;
     } else if (p.lse != nullptr) {
-      p.lse[row0 + tid] = sum > 0.0f ? s_big[tid] + logf(sum) : -INFINITY;
+      p.lse[row0 + tid] = sum == 0.0f ? -INFINITY : s_big[tid] + logf(sum);
     }
   }
 }
