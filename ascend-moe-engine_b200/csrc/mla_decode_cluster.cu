@@ -298,7 +298,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 
   const uint32_t tmem = misc->tmem_base;
   bool ok = true;
-  float m_run[2] = {-INFINITY, -INFINITY};  // reference maxima of this thread's two rows, log2 domain
+  float m_run[2] = {kLowest, kLowest};  // reference maxima of this thread's two rows, log2 domain
   float l_run[2] = {0.0f, 0.0f};
 
   if (warp == 4 && n > 0) {
@@ -639,12 +639,12 @@ __global__ void __launch_bounds__(kThreads, 1)
         const float tile_max = raw_max * p.scale_log2;
         const bool moves = tile_max > m_run[r] + kRescaleThreshold;
         const float m_new = moves ? tile_max : m_run[r];
-        const float factor = i == 0 || !moves ? 1.0f : ptx::Ex2Approx(m_run[r] - m_new);
+        const float factor = i == 0 ? 1.0f : ptx::Ex2Approx(m_run[r] - m_new);
         m_run[r] = m_new;
         rescale |= moves && i > 0;
         if ((lane & 3) == 0) misc->factor[head0 + 8 * r] = factor;
         l_run[r] *= factor;
-        neg_m[r] = m_new == -INFINITY ? 0.0f : -m_new;  // (as long as every score was -infinity, weights are zero)
+        neg_m[r] = -m_run[r];
       }
       uint32_t packed[2][8], packed_lo[2][kSplitP ? 8 : 1];
 #pragma unroll

@@ -801,7 +801,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     bool first_segment_of_cta = true;
 
     while (ok && walk.Next(&seq, &t_lo, &t_hi, &seq_tiles, &seq_len)) {
-      float m_run[2] = {-INFINITY, -INFINITY};  // reference maxima of the two rows, log2 domain (s * scale * log2e)
+      float m_run[2] = {kLowest, kLowest};  // reference maxima of the two rows, log2 domain (s * scale * log2e)
       float l_run[2] = {0.0f, 0.0f};
       const int n = t_hi - t_lo;
       // The four warps leave this loop, and the segment, on the same vote: a wait can run out for one of them and not for
@@ -857,7 +857,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           raw_max[r] = fmaxf(raw_max[r], __shfl_xor_sync(0xffffffffu, raw_max[r], 2));
           const float tile_max = raw_max[r] * p.scale_log2;
           // The reference maximum moves only when the tile's exceeds it by the threshold (always on a segment's
-          // first tile, where m_run is -inf and nothing has been accumulated). No branch: a factor of
+          // first tile, where nothing has been accumulated). No branch: a factor of
           // exp2(0) = 1 costs one more EX2, a divergent branch costs more.
           const bool moves = tile_max > m_run[r] + kRescaleThreshold;
           const float m_new = moves ? tile_max : m_run[r];
@@ -972,7 +972,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           p.user_m[static_cast<int64_t>(seq) * kHeads + head] = m_nat;
           p.user_l[static_cast<int64_t>(seq) * kHeads + head] = l_row;
         } else if (p.lse != nullptr) {
-          p.lse[static_cast<int64_t>(seq) * kHeads + head] = m_nat + logf(l_row);
+          p.lse[static_cast<int64_t>(seq) * kHeads + head] = l_row == 0.0f ? -INFINITY : m_nat + logf(l_row);
         }
       }
       if (ptx::NamedBarrierOr(1, kSoftmaxThreads, !ok)) {

@@ -25,6 +25,8 @@ constexpr int kSoftmaxWarps = kSoftmaxThreads / 32;     // one lane of each arri
 constexpr uint32_t kTmemCols = 512;
 constexpr uint32_t kTmemColS = 256;                     // S buffers at columns 256 and 256 + kTile
 constexpr float kRescaleThreshold = 8.0f;               // log2 units: rescale O only when max grows by > 2^8
+// Where running maxima start: finite, so that subtracting one from a score of -infinity leaves -infinity, a weight of zero.
+constexpr float kLowest = -3.4028234663852886e38f;
 
 __device__ __forceinline__ int TilesOf(int len) { return (len + kTile - 1) / kTile; }
 
