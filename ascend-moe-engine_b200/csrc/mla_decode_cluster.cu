@@ -113,6 +113,7 @@ struct ClusterParams {
   int32_t block_size;
   int32_t stable_tables;
   float scale_log2;
+  float nat_hi, nat_lo;  // scale / scale_log2 in two terms: from the kernel's log2 domain back to natural logarithms
   __nv_bfloat16* out;
   uint8_t* out_q;
   uint8_t* out_scale;
@@ -778,12 +779,13 @@ __global__ void __launch_bounds__(kThreads, 1)
   auto emit_ml = [&](int h, float big, float total) {  // head h of this CTA's
     if (first + h >= p.heads) return;
     const int64_t at = static_cast<int64_t>(seq) * p.heads + first + h;
-    const float m_nat = big * 0.6931471805599453f;
+    // (The weights are exp2(s * scale_log2 - big) with scale_log2 rounded once; going back by the quotient of the two scales,
+    // and rounding once more at the end, the log-sum-exp is as close to the scores' as with natural exponentials.)
     if (want_partial) {
-      p.user_m[at] = m_nat;
+      p.user_m[at] = big == -INFINITY ? big : fmaf(big, p.nat_hi, big * p.nat_lo);
       p.user_l[at] = total;
     } else if (p.lse != nullptr) {
-      p.lse[at] = total == 0.0f ? -INFINITY : m_nat + logf(total);
+      p.lse[at] = total == 0.0f ? -INFINITY : fmaf(big, p.nat_hi, fmaf(big, p.nat_lo, logf(total)));
     }
   };
   // (m, l) of this CTA's token range: lane j < 16 of a softmax warp takes row j of the warp's sixteen.
@@ -1102,6 +1104,9 @@ int32_t Launch(const b200kv_decode_args& a, int source, bool split_p, int32_t cl
   p.block_size = a.block_size;
   p.stable_tables = (a.flags & B200KV_DECODE_STABLE_TABLES) != 0 ? 1 : 0;
   p.scale_log2 = a.scale * 1.4426950408889634f;
+  const double nat = static_cast<double>(a.scale) / static_cast<double>(p.scale_log2);
+  p.nat_hi = static_cast<float>(nat);
+  p.nat_lo = static_cast<float>(nat - static_cast<double>(p.nat_hi));
   p.out = static_cast<__nv_bfloat16*>(a.out);
   p.out_q = static_cast<uint8_t*>(a.out_fp8);
   p.out_scale = static_cast<uint8_t*>(a.out_scale);

@@ -240,3 +240,22 @@ def test_scores_of_minus_infinity_have_no_weight(kv_len, bs, heads):
     pool[rows[hit], 575] = float("inf")
     out, lse = _decode_dev(q, pool, table, lens, bs)
     assert (out[hit] == 0).all() and (lse[hit] == float("-inf")).all()
+
+
+@pytest.mark.parametrize("gain", [1.0, 3.0])
+def test_log_sum_exp_of_any_geometry_is_as_exact_as_the_cuda_core_kernels(gain):
+    """Against float64, over lengths, head counts and block sizes together: the root mean square of the tensor cores' sums
+    and of the fp32 chains differ by the luck of their roundings (both are close to that of the fp32 result itself), so by
+    less than a tenth."""
+    squares = {b200kv.DECODE_AUTO: [], b200kv.DECODE_SIMT: []}
+    for seed in range(3):
+        for kv_len in ([1, 17, 64, 65, 1000, 333], [4096, 3000], [8192]):
+            for heads, bs in ((64, 16), (64, 1), (16, 64), (128, 8)):
+                q, pool, table, lens, rows = _case(kv_len, bs, heads, seed)
+                q = (q.float() * gain).bfloat16()
+                _, want = _attention_f64(q, pool, rows)
+                for variant, errors in squares.items():
+                    _, lse = _decode_dev(q, pool, table, lens, bs, variant)
+                    errors.append((lse.double() - want).pow(2).mean(1))
+    auto, simt = (torch.cat(squares[v]).mean().sqrt().item() for v in (b200kv.DECODE_AUTO, b200kv.DECODE_SIMT))
+    assert auto <= 1.1 * simt, (auto, simt)
