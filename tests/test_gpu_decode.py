@@ -207,13 +207,14 @@ def test_decode_reports_bad_block_without_faulting():
     table = np.array([[1, 99]], dtype=np.int32)
     q = kvo.make_q(1)
     from gpu_util import to_dev_bf16, to_dev_i32
-    for variant in (b200kv.DECODE_SIMT, b200kv.DECODE_TCGEN05):
+    # (a grid limit keeps a call on the kernel for many tiles)
+    for variant, max_ctas in ((b200kv.DECODE_SIMT, 0), (b200kv.DECODE_TCGEN05, 0), (b200kv.DECODE_TCGEN05, 3)):
         qd, pd = to_dev_bf16(q), to_dev_bf16(pool)
         out = torch.zeros((1, 64, 512), dtype=torch.bfloat16, device="cuda")
-        ws = torch.empty(b200kv.decode_workspace_bytes(1), dtype=torch.uint8, device="cuda")
+        ws = torch.empty(b200kv.decode_workspace_bytes(1, 64, max_ctas), dtype=torch.uint8, device="cuda")
         status = b200kv.new_status()
         b200kv.mla_decode(qd, b200kv.pool_view(pd), to_dev_i32(table), to_dev_i32([100]), bs, 1.0 / 24.0, out=out,
-                          workspace=ws, variant=variant, status=status)
+                          workspace=ws, variant=variant, max_ctas=max_ctas, status=status)
         torch.cuda.synchronize()
         st = status.cpu().tolist()
         assert st[0] == b200kv.DEV_BAD_BLOCK and st[1] == 0 and st[2] == 1 and st[3] == 99
@@ -309,10 +310,10 @@ def test_gathered_rows_outside_the_pool_are_recorded_not_read():
     rows[1, 7] = pool_rows  # one past the end
     out = torch.zeros((2, 64, 512), dtype=torch.bfloat16, device="cuda")
     ws = torch.empty(b200kv.decode_workspace_bytes(2, 64, 0), dtype=torch.uint8, device="cuda")
-    for variant in (b200kv.DECODE_TCGEN05, b200kv.DECODE_SIMT):
+    for variant, max_ctas in ((b200kv.DECODE_TCGEN05, 0), (b200kv.DECODE_TCGEN05, 3), (b200kv.DECODE_SIMT, 0)):
         status = b200kv.new_status()
         b200kv.mla_decode(q, b200kv.pool_view(pool), None, to_dev_i32(np.array([64, 64], dtype=np.int32)), 64, 1.0 / 24.0,
-                          out=out, workspace=ws, variant=variant, status=status, row_index=to_dev_i32(rows))
+                          out=out, workspace=ws, variant=variant, max_ctas=max_ctas, status=status, row_index=to_dev_i32(rows))
         torch.cuda.synchronize()
         assert status.cpu().tolist()[0] == b200kv.DEV_BAD_BLOCK
     with pytest.raises(b200kv.B200KVError) as err:  # a row list and a KV range exclude each other
@@ -578,8 +579,8 @@ def test_fused_append_through_a_bad_table_entry_writes_nothing():
         assert np.array_equal(from_dev_bf16(pool), want_pool), "a pool row other than sequence 0's slot changed"
 
 
-@pytest.mark.parametrize("variant", VARIANTS)
-def test_length_beyond_the_table_row_is_reported_not_read(variant):
+@pytest.mark.parametrize("variant,max_ctas", [(b200kv.DECODE_SIMT, 0), (b200kv.DECODE_TCGEN05, 0), (b200kv.DECODE_TCGEN05, 3)])
+def test_length_beyond_the_table_row_is_reported_not_read(variant, max_ctas):
     """kv_len lives on the device, so the host cannot check it against max_blocks * block_size: a length that
     runs past the sequence's row of the block table is recorded as a bad block, and the entries of the next
     row (or the memory behind the table) are never used as block ids."""
@@ -590,10 +591,10 @@ def test_length_beyond_the_table_row_is_reported_not_read(variant):
     table = np.array([[1, 2], [3, 4]], dtype=np.int32)
     for seq, lens in ((0, [3 * bs, 10]), (1, [10, 2 * bs + 1])):
         out = torch.zeros((2, 64, 512), dtype=torch.bfloat16, device="cuda")
-        ws = torch.empty(b200kv.decode_workspace_bytes(2), dtype=torch.uint8, device="cuda")
+        ws = torch.empty(b200kv.decode_workspace_bytes(2, 64, max_ctas), dtype=torch.uint8, device="cuda")
         status = b200kv.new_status()
         b200kv.mla_decode(to_dev_bf16(kvo.make_q(2)), b200kv.pool_view(pool), to_dev_i32(table), to_dev_i32(lens), bs,
-                          1.0 / 24.0, out=out, workspace=ws, variant=variant, status=status)
+                          1.0 / 24.0, out=out, workspace=ws, variant=variant, max_ctas=max_ctas, status=status)
         torch.cuda.synchronize()
         st = status.cpu().tolist()
         assert st[0] == b200kv.DEV_BAD_BLOCK and st[1] == seq and st[2] == 2 and st[3] == -1, st

@@ -1,5 +1,5 @@
 """The cluster form of the decode attention (one launch, partials exchanged through distributed shared memory): every
-cluster size (the batch decides it), every split of a cluster into token and column ranges (the length decides it),
+cluster size (the batch decides it), every split of a cluster into token ranges and head groups (the length decides it),
 tile edges, and the geometries that only this form serves on tensor cores (any block size, any head count)."""
 import numpy as np
 import pytest
@@ -50,7 +50,8 @@ def test_small_batches_match_the_reference(batch):
 
 @pytest.mark.parametrize("length", [1, 64, 100, 129, 257, 512, 513, 1024, 2048, 8192])
 def test_one_sequence_of_every_split(length):
-    """Up to 8,192 tokens one sequence takes a cluster of 16: 4 x 4, 8 x 2 and 16 x 1 token x column ranges."""
+    """Up to 2,048 tokens one sequence takes a cluster of 16: 4 x 4, 8 x 2 and 16 x 1 token ranges x head groups (8,192 are the
+    other kernel's)."""
     kv_len = np.array([length], dtype=np.int32)
     pool, poisoned, table = _pool_with_poison(kv_len, 128)
     q = kvo.make_q(1)
@@ -64,8 +65,8 @@ def test_one_sequence_of_every_split(length):
 
 @pytest.mark.parametrize("kv_len", [[1], [129], [64, 65, 1, 700], [128] * 40])
 def test_fused_append_and_quantisation(kv_len):
-    """The CTAs of every column range write the new row before they load its tile; the quantised bytes are those of the
-    stand-alone quantiser on the output."""
+    """The CTAs of every head group put the new row into their copy of its tile, one of them into the pool; the quantised
+    bytes are those of the stand-alone quantiser on the output."""
     bs, batch = 64, len(kv_len)
     kv_len = np.array(kv_len, dtype=np.int32)
     pool, _, table = _pool_with_poison(kv_len, bs)
@@ -259,3 +260,94 @@ def test_log_sum_exp_of_any_geometry_is_as_exact_as_the_cuda_core_kernels(gain):
                     errors.append((lse.double() - want).pow(2).mean(1))
     auto, simt = (torch.cat(squares[v]).mean().sqrt().item() for v in (b200kv.DECODE_AUTO, b200kv.DECODE_SIMT))
     assert auto <= 1.1 * simt, (auto, simt)
+
+
+@pytest.mark.parametrize("batch,longest", [(40, 750), (140, 512)])
+def test_fused_append_where_a_cta_has_several_tiles(batch, longest):
+    """The new row goes into a stage that has been filled before; bf16 output alone (quantised calls come here with a tile a
+    CTA only). Rows at the beginning, in the middle and at the end of tiles; the pool bit for bit."""
+    bs = 64
+    kv_len = np.array([[longest, longest // 64 * 64, longest // 64 * 64 - 63, 300, 449, 129, 1, 64, 65, 257][i % 10] for i in range(batch)], dtype=np.int32)
+    pool, poisoned, table = _pool_with_poison(kv_len, bs)
+    latent, rope = kvo.normal_bf16(batch * 512, 21).reshape(batch, 512), kvo.normal_bf16(batch * 64, 22).reshape(batch, 64)
+    last = kv_len.astype(np.int64) - 1
+    rows = table[np.arange(batch), last // bs].astype(np.int64) * bs + last % bs
+    whole, want = pool.copy(), poisoned.copy()
+    for p in (whole, want):
+        p[rows, :512], p[rows, 512:] = latent, rope
+    q = kvo.make_q(batch)
+    ref_out, ref_lse = scenarios.ref_attention_f64(q, whole, table, kv_len, bs, 1.0 / 24.0)
+    for max_ctas in (0, 5):  # and the kernel for many tiles
+        d_pool, status = to_dev_bf16(poisoned), b200kv.new_status()
+        out = torch.empty((batch, 64, 512), dtype=torch.bfloat16, device="cuda")
+        lse = torch.empty((batch, 64), dtype=torch.float32, device="cuda")
+        ws = torch.empty(b200kv.decode_workspace_bytes(batch, 64, max_ctas), dtype=torch.uint8, device="cuda")
+        b200kv.mla_decode(to_dev_bf16(q), b200kv.pool_view(d_pool), to_dev_i32(table), to_dev_i32(kv_len), bs, 1.0 / 24.0, out=out, lse=lse,
+                          workspace=ws, status=status, new_rows=(to_dev_bf16(latent), to_dev_bf16(rope)), max_ctas=max_ctas)
+        status_ok(status)
+        assert np.array_equal(from_dev_bf16(d_pool), want)
+        scenarios.check_attention(from_dev_bf16(out), lse.cpu().numpy(), ref_out, ref_lse, what=f"append, several tiles, max_ctas {max_ctas}")
+
+
+@pytest.mark.parametrize("heads,bs", [(64, 16), (64, 48), (16, 64), (16, 16), (65, 1)])
+@pytest.mark.parametrize("two_arrays", [False, True])
+def test_shards_and_strided_queries_of_any_geometry(heads, bs, two_arrays):
+    """Shards that begin anywhere (out and lse of a range that starts past the first tokens), queries that are slices of wider
+    rows with the heads outermost, and latent and rope in arrays of their own."""
+    begin = np.array([0, 48, 100, 1, 333], dtype=np.int32)
+    length = np.array([64, 200, 1, 0, 700], dtype=np.int32)
+    pool, _, table = _pool_with_poison(begin + np.maximum(length, 1), bs)
+    q = kvo.make_q(len(length), heads=heads, scale=0.3)
+    ref_out, ref_lse = scenarios.ref_attention_f64(q, pool, table, length, bs, 1.0 / 24.0, kv_begin=begin)
+    d_pool = to_dev_bf16(pool)
+    wide = torch.full((len(pool), 640), float("nan"), dtype=torch.bfloat16, device="cuda")
+    wide[:, :512] = d_pool[:, :512]
+    rope = d_pool[:, 512:].contiguous()
+    view = b200kv.pool_view(wide[:, :512], rope) if two_arrays else b200kv.pool_view(d_pool)
+    by_head = torch.full((heads, len(length), 640), float("nan"), dtype=torch.bfloat16, device="cuda")
+    by_head[:, :, 64:] = to_dev_bf16(q).transpose(0, 1)
+    d_q = by_head.transpose(0, 1)[:, :, 64:]
+    out = torch.full((len(length), heads, 512), float("nan"), dtype=torch.bfloat16, device="cuda")
+    lse = torch.full((len(length), heads), float("nan"), dtype=torch.float32, device="cuda")
+    status = b200kv.new_status()
+    ws = torch.empty(b200kv.decode_workspace_bytes(len(length), heads), dtype=torch.uint8, device="cuda")
+    b200kv.mla_decode(d_q, view, to_dev_i32(table), to_dev_i32(length), bs, 1.0 / 24.0, out=out, lse=lse, kv_begin=to_dev_i32(begin),
+                      workspace=ws, status=status)
+    status_ok(status)
+    scenarios.check_attention(from_dev_bf16(out), lse.cpu().numpy(), ref_out, ref_lse, what=f"shards {heads} x {bs}")
+
+
+@pytest.mark.parametrize("bs", [16, 48, 1])
+def test_quantised_output_of_any_block_size(bs):
+    """The quantised bytes are those of the stand-alone quantiser on the output, and of the CUDA-core path's wherever the two
+    kernels' bf16 agree on a block of 32."""
+    kv_len = np.array([1, 70, 1000, 0, 333], dtype=np.int32)
+    pool, _, table = _pool_with_poison(kv_len, bs)
+    q, batch = to_dev_bf16(kvo.make_q(len(kv_len))), len(kv_len)
+    ws = torch.empty(b200kv.decode_workspace_bytes(batch), dtype=torch.uint8, device="cuda")
+    got = []
+    for variant in (b200kv.DECODE_AUTO, b200kv.DECODE_SIMT):
+        out = torch.empty((batch, 64, 512), dtype=torch.bfloat16, device="cuda")
+        fp8 = torch.empty((batch, 64, 512), dtype=torch.uint8, device="cuda")
+        scales = torch.empty((batch, 64, 16), dtype=torch.uint8, device="cuda")
+        status = b200kv.new_status()
+        b200kv.mla_decode(q, b200kv.pool_view(to_dev_bf16(pool)), to_dev_i32(table), to_dev_i32(kv_len), bs, 1.0 / 24.0, out=out, workspace=ws,
+                          status=status, variant=variant, quantised=(fp8, scales))
+        status_ok(status)
+        fp8_2, scales_2 = torch.empty((batch, 64 * 512), dtype=torch.uint8, device="cuda"), torch.empty((batch, 1024), dtype=torch.uint8, device="cuda")
+        b200kv.mx_quant_e4m3(out.view(batch, -1), fp8_2, scales_2)
+        assert torch.equal(fp8.view(batch, -1), fp8_2) and torch.equal(scales.view(batch, -1), scales_2)
+        got.append((out.view(-1, 32), fp8.view(-1, 32)))
+    same = (got[0][0] == got[1][0]).all(1)
+    assert same.float().mean() > 0.8 and torch.equal(got[0][1][same], got[1][1][same])
+
+
+def test_two_sequences_of_up_to_4096_tokens():
+    """The longest sequences that clusters of sixteen take (two of 64 tiles), and one tile more, which they do not."""
+    for longest in (2049, 3000, 4096, 4160):
+        kv_len = [longest, longest - 777]
+        q, pool, table, lens, rows = _case(kv_len, 64)
+        want, want_lse = _attention_f64(q, pool, rows)
+        out, lse = _decode_dev(q, pool, table, lens, 64)
+        assert ((out.double() - want).abs() <= 2e-3 + 1e-2 * want.abs().amax(dim=2, keepdim=True)).all()
+        assert (lse.double() - want_lse).abs().max() <= 1e-4
