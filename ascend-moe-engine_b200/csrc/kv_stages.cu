@@ -177,8 +177,8 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, 4) RotateKernel(ProducerPar
 // us for 16,384 / 49,157 / 131,072 rows: 11.3 / 28.4 / 68.2 before (4.9 TB/s), 10.9 / 26.2 / 63.1 without reading ahead,
 // 12.1 / 24.4 / 57.5 with eight CTAs an SM in the grid, 8.5 / 22.9 / 55.9 (6.0 TB/s) so.
 constexpr int kResidentCtas = 2;
-// kVectors: the launch also rotates the query's vectors, eight a pass (calls of a few tokens).
-template <bool kVectors>
+// kVectors: the launch also rotates the query's vectors, so many times eight a pass (calls of up to some thousand tokens).
+template <int kVectors>
 __global__ void __launch_bounds__(kWarpsPerCta * 32, kResidentCtas) ProducerKernel(ProducerParams p) {
   GridDependencyTrigger();
   GridDependencyWait();
@@ -187,8 +187,9 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, kResidentCtas) ProducerKern
   const int64_t n_warps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
   const int64_t rows = p.tokens;
   const int64_t row_items = (rows + kRowsPerPass - 1) / kRowsPerPass;
-  const int64_t vectors = kVectors ? p.tokens * p.heads : 0;
-  const int64_t vector_items = (vectors + 7) / 8;
+  constexpr int kItemVectors = kVectors > 0 ? 8 * kVectors : 8;
+  const int64_t vectors = kVectors > 0 ? p.tokens * p.heads : 0;
+  const int64_t vector_items = (vectors + kItemVectors - 1) / kItemVectors;
   // gamma of this lane's columns 8 lane .. + 7 and 256 + 8 lane .. + 7
   const uint4 ga = *reinterpret_cast<const uint4*>(p.gamma + 8 * lane), gb = *reinterpret_cast<const uint4*>(p.gamma + 256 + 8 * lane);
   const uint32_t gamma[8] = {ga.x, ga.y, ga.z, ga.w, gb.x, gb.y, gb.z, gb.w};
@@ -226,9 +227,11 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, kResidentCtas) ProducerKern
   };
   if (warp < row_items) read(warp);
   for (int64_t item = warp; item < row_items + vector_items; item += n_warps) {
-    if (kVectors && item >= row_items) {
-      RotateVectors<1>(p, (item - row_items) * 8, vectors);
-      continue;
+    if constexpr (kVectors > 0) {
+      if (item >= row_items) {
+        RotateVectors<kVectors>(p, (item - row_items) * kItemVectors, vectors);
+        continue;
+      }
     }
     const int64_t t0 = item * kRowsPerPass;
     const int64_t t = t0 + half;  // this half-warp's row
@@ -389,15 +392,20 @@ int32_t LaunchProducer(const ProducerParams& p, void* stream, const char* what) 
     return dim3(static_cast<unsigned>(want < cap ? want : cap));
   };
   const int64_t row_items = (rows + kRowsPerPass - 1) / kRowsPerPass, vector_items = (vectors + 7) / 8;
-  // One launch up to four passes a warp; beyond that the vectors get a kernel of their own, with twice the warps on an SM.
-  // 256 / 512 / 1,024 / 4,096 tokens x 64 heads in one launch 3.0 / 3.9 / 5.95 / 20.0 us, in two 4.35 / 4.75 / 6.75 / 15.0
-  // (before, in one: 4.3 / 4.45 / 5.95 / 17.1); 1,024 are 3.7 passes.
-  if (rows > 0 && vectors > 0 && row_items + vector_items <= 4 * sms * kResidentCtas * kWarpsPerCta) {
-    return CheckCuda(LaunchOverlapped(ProducerKernel<true>, grid_for(row_items + vector_items, sms * kResidentCtas),
+  // One launch up to seven and three quarters passes a warp; beyond that the vectors get a kernel of their own, with twice the
+  // warps on an SM. Two rounds of vectors a pass cost one and a half times as much as one, so they pay where they make the
+  // passes fewer by more. us for 1,024 / 1,536 / 2,048 / 2,300 tokens x 64 heads (3.7 .. 8.3 passes) in one launch with one
+  // round 5.70 / 7.54 / 9.35 / 10.3, with two 4.96 / 6.38 / 7.87 / 9.41, in two launches 6.53 / 8.56 / 8.85 / 8.85 (one kernel
+  // of 64 registers, before: 5.79 / 7.42 / 8.29 / 9.66).
+  const int64_t resident = sms * kResidentCtas * kWarpsPerCta;
+  if (rows > 0 && vectors > 0 && 4 * (row_items + vector_items) <= 31 * resident) {
+    const int64_t one = row_items + vector_items, two = row_items + (vectors + 15) / 16;
+    const bool rounds_of_two = 2 * ((one + resident - 1) / resident) > 3 * ((two + resident - 1) / resident);
+    return CheckCuda(LaunchOverlapped(rounds_of_two ? ProducerKernel<2> : ProducerKernel<1>, grid_for(rounds_of_two ? two : one, sms * kResidentCtas),
                                       dim3(kWarpsPerCta * 32), 0, st, p), what);
   }
   if (rows > 0) {
-    if (int32_t rc = CheckCuda(LaunchOverlapped(ProducerKernel<false>, grid_for(row_items, sms * kResidentCtas), dim3(kWarpsPerCta * 32), 0, st,
+    if (int32_t rc = CheckCuda(LaunchOverlapped(ProducerKernel<0>, grid_for(row_items, sms * kResidentCtas), dim3(kWarpsPerCta * 32), 0, st,
                                                p), what)) return rc;
   }
   if (vectors == 0) return B200KV_OK;

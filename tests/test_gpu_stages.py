@@ -522,10 +522,10 @@ def test_indexer_operator_through_the_operator_abi():
                                     eps_rel=1e-6)
 
 
-@pytest.mark.parametrize("tokens,heads", [(31, 63), (593, 64), (1025, 64), (1203, 63), (2, 5000)])
+@pytest.mark.parametrize("tokens,heads", [(31, 63), (593, 64), (701, 32), (1025, 64), (1203, 63), (1801, 16), (2155, 64), (2165, 64), (2, 5000)])
 def test_query_rotation_in_its_own_kernel(tokens, heads):
-    """Query slices that share the rows' launch and those that get their own (from four passes a warp on), with one and
-    two rounds a warp, on both sides of each line; slices of wider rows, so that the rest has to stay as it is."""
+    """Query slices that share the rows' launch, with one and with two rounds of vectors a pass, and those that get their own
+    (from seven and three quarters passes a warp on), on both sides of each line; slices of wider rows, so that the rest has to stay as it is."""
     rows = tokens + 64
     kv_a = kvo.normal_bf16(tokens * 576, 3).reshape(tokens, 576)
     gamma, (cos, sin) = gamma_bits(), rope_tables(tokens, first_pos=11)
