@@ -546,11 +546,17 @@ __global__ void __launch_bounds__(kSortThreads) IndexerSelectKernel(SelectParams
 }
 
 int32_t LaunchSelect(SelectParams p, int32_t batch, int64_t max_kv_len, cudaStream_t stream) {
-  // How many clusters of 1, 2, 4, 8, 16 CTAs the device holds at once; looked up once per thread and device.
-  static thread_local int known_device = -1;
-  static thread_local int32_t most[5];
+  // How many clusters of 1, 2, 4, 8, 16 CTAs a device holds at once; looked up once per thread and device (a device number
+  // beyond the table whenever it comes after another).
+  constexpr int kKnownDevices = 16;
+  struct Limits {
+    int device = -1;
+    int32_t most[5] = {};
+  };
+  static thread_local Limits known[kKnownDevices];
   int device = 0;
   if (int32_t rc = CheckCuda(cudaGetDevice(&device), "cudaGetDevice")) return rc;
+  Limits& limits = known[device % kKnownDevices];
   cudaLaunchConfig_t config = {};
   config.blockDim = dim3(kSortThreads);
   config.dynamicSmemBytes = sizeof(SelectShared);
@@ -562,7 +568,7 @@ int32_t LaunchSelect(SelectParams p, int32_t batch, int64_t max_kv_len, cudaStre
   attrs[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attrs[1].val.programmaticStreamSerializationAllowed = 1;
   config.attrs = attrs;
-  if (device != known_device) {
+  if (device != limits.device) {
     if (int32_t rc = CheckCuda(cudaFuncSetAttribute(IndexerSelectKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(SelectShared))), "indexer top-k smem opt-in")) return rc;
     if (int32_t rc = CheckCuda(cudaFuncSetAttribute(IndexerSelectKernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1), "indexer top-k cluster opt-in")) return rc;
     for (int i = 0; i < 5; ++i) {
@@ -574,13 +580,13 @@ int32_t LaunchSelect(SelectParams p, int32_t batch, int64_t max_kv_len, cudaStre
         cudaGetLastError();  // a size the device does not offer
         clusters = 0;
       }
-      most[i] = clusters;
+      limits.most[i] = clusters;
     }
-    known_device = device;
+    limits.device = device;
   }
   int size = 0;
   while (size < 4 && max_kv_len > static_cast<int64_t>(kTokensPerCta) << size) ++size;
-  while (size > 0 && batch > most[size]) --size;
+  while (size > 0 && batch > limits.most[size]) --size;
   p.cluster_log2 = size;
   attrs[0].val.clusterDim.x = 1u << size;
   config.gridDim = dim3(static_cast<unsigned>(batch) << size);  // (in x, which has room for any batch)

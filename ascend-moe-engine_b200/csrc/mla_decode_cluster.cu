@@ -1015,16 +1015,19 @@ cudaLaunchConfig_t ConfigOf(int32_t cluster, int32_t seqs, int32_t head_groups, 
 }
 
 // How many clusters of 1, 2, 4, 8, 16 CTAs the current device holds at once (index: log2 of the size), and the
-// kernels' opt-ins; looked up once per thread and device.
+// kernels' opt-ins; looked up once per thread and device (a thread that goes from device to device keeps them all; a device
+// number beyond the table is looked up whenever it comes after another).
 struct ClusterLimits {
   int device = -1;
   int32_t most[5] = {};
 };
+constexpr int kKnownDevices = 16;
 
 int32_t LimitsOf(const ClusterLimits** out) {
-  static thread_local ClusterLimits limits;
+  static thread_local ClusterLimits known[kKnownDevices];
   int device = 0;
   if (int32_t rc = CheckCuda(cudaGetDevice(&device), "cudaGetDevice")) return rc;
+  ClusterLimits& limits = known[device % kKnownDevices];
   if (device != limits.device) {
     const struct {
       ClusterKernel kernel;
