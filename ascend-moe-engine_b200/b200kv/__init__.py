@@ -242,10 +242,8 @@ _mla_decode, _mla_decode_static = _packed_entry("b200kv_mla_decode"), _packed_en
 _append_fused, _indexer_topk = _packed_entry("b200kv_append_fused"), _packed_entry("b200kv_indexer_topk")
 
 
-def _view_bytes(view: PoolView) -> bytes:
-    if not isinstance(view, PoolView):
-        raise TypeError(f"expected a PoolView, got {type(view).__name__}")
-    return bytes(view)
+def _refuse_view(view):
+    raise TypeError(f"expected a PoolView, got {type(view).__name__}")
 
 
 def _stream_handle(stream=None) -> int:
@@ -294,7 +292,7 @@ def append(view: PoolView, latent_src, rope_src, slot_mapping, status=None, stre
     slot_mapping int32 [T] on the device."""
     n = slot_mapping.shape[0]
     check(lib.b200kv_append(ctypes.byref(view), _ptr(latent_src), latent_src.stride()[0] if n else LATENT_DIM,
-                            _ptr(rope_src), rope_src.stride()[0] if n else ROPE_DIM, _ptr(slot_mapping), n,
+                            _ptr(rope_src), rope_src.stride()[0] if n else ROPE_DIM, slot_mapping.data_ptr(), n,
                             _stream_handle(stream), _ptr(status)))
 
 
@@ -312,7 +310,7 @@ def append_fused(view: PoolView, kv_a, gamma, cos, sin, slot_mapping, eps: float
     latent_ptr, latent_stride = (0, 0) if latent_out is None else (latent_out.data_ptr(), latent_out.stride()[0])
     rope_ptr, rope_stride = (0, 0) if rope_out is None else (rope_out.data_ptr(), rope_out.stride()[0])
     cos_stride, sin_stride = cos.stride(), sin.stride()
-    a = _pack_producer(_view_bytes(view), _ptr(kv_a), kv_a.stride()[0] if n else LATENT_DIM + ROPE_DIM, _ptr(gamma), eps,
+    a = _pack_producer(bytes(view) if isinstance(view, PoolView) else _refuse_view(view), _ptr(kv_a), kv_a.stride()[0] if n else LATENT_DIM + ROPE_DIM, _ptr(gamma), eps,
                      cos.data_ptr(), cos_stride[0] if len(cos_stride) == 2 else 0,
                      sin.data_ptr(), sin_stride[0] if len(sin_stride) == 2 else 0, slot_mapping.data_ptr(), n,
                      q_ptr, q_token_stride, q_head_stride, heads, latent_ptr, latent_stride, rope_ptr, rope_stride,
@@ -323,7 +321,7 @@ def append_fused(view: PoolView, kv_a, gamma, cos, sin, slot_mapping, eps: float
 def mx_quant_e4m3(x, q, scales, stream=None) -> None:
     """x bf16 [rows, cols] -> q uint8 [rows, cols] (FP8 E4M3 codes), scales uint8 [rows, cols / 32] (E8M0)."""
     rows, cols = x.shape[0], x.shape[1]
-    check(lib.b200kv_mx_quant_e4m3(_ptr(x), x.stride()[0], rows, cols, _ptr(q), q.stride()[0], _ptr(scales),
+    check(lib.b200kv_mx_quant_e4m3(x.data_ptr(), x.stride()[0], rows, cols, q.data_ptr(), q.stride()[0], scales.data_ptr(),
                                    scales.stride()[0], _stream_handle(stream)))
 
 
@@ -331,7 +329,7 @@ def gather(view: PoolView, block_table, kv_len, block_size: int, out_latent, out
            total_rows: int, status=None, stream=None) -> None:
     batch = kv_len.shape[0]
     check(lib.b200kv_gather(ctypes.byref(view), _ptr(block_table), block_table.stride()[0] if batch else 1,
-                            _ptr(kv_len), batch, block_size, _ptr(out_latent),
+                            kv_len.data_ptr(), batch, block_size, _ptr(out_latent),
                             out_latent.stride()[0] if total_rows else LATENT_DIM, _ptr(out_rope),
                             out_rope.stride()[0] if total_rows else ROPE_DIM, _ptr(out_row_offsets), total_rows,
                             _stream_handle(stream), _ptr(status)))
@@ -350,8 +348,8 @@ def indexer_topk(q_fp8, q_scale, weights, key_pool, k_scale, block_table, kv_len
     index = torch.empty((batch, k), dtype=torch.int32, device=q_fp8.device)
     n_sel = torch.empty((batch,), dtype=torch.int32, device=q_fp8.device)
     ws = torch.empty(lib.b200kv_indexer_workspace_bytes(batch, max_kv_len), dtype=torch.uint8, device=q_fp8.device)
-    a = _pack_indexer(_ptr(q_fp8), _ptr(q_scale), _ptr(weights), heads, _ptr(key_pool), key_pool.stride()[0],
-                    _ptr(k_scale), key_pool.shape[0], _ptr(block_table), block_table.shape[1], _ptr(kv_len),
+    a = _pack_indexer(q_fp8.data_ptr(), _ptr(q_scale), _ptr(weights), heads, key_pool.data_ptr(), key_pool.stride()[0],
+                    _ptr(k_scale), key_pool.shape[0], block_table.data_ptr(), block_table.shape[1], _ptr(kv_len),
                     batch, block_size, max_kv_len, k, index.data_ptr(), n_sel.data_ptr(), ws.data_ptr(), ws.numel(), variant,
                     _ptr(rows_out))
     check(_indexer_topk(a, _stream_handle(stream), _ptr(status)))
@@ -402,17 +400,19 @@ def _decode_args(q, view: PoolView, block_table, kv_len, block_size: int, scale:
     batch, heads = q.shape[:2]
     q_seq_stride, q_head_stride = q.stride()[:2]
     table, max_blocks = (0, 0) if block_table is None else (block_table.data_ptr(), block_table.stride()[0])
-    o, m, l = (0, 0, 0) if partial is None else (_ptr(t) for t in partial)
+    o = m = l = 0
+    if partial is not None:
+        o, m, l = (_ptr(t) for t in partial)
     ws, ws_bytes = (0, 0) if workspace is None else (workspace.data_ptr(), workspace.nbytes)
     if new_rows is None:
         latent = latent_stride = rope = rope_stride = 0
     else:
         new_latent, new_rope = new_rows
-        latent, latent_stride = _ptr(new_latent), new_latent.stride()[0]
-        rope, rope_stride = _ptr(new_rope), new_rope.stride()[0]
+        latent, latent_stride = new_latent.data_ptr(), new_latent.stride()[0]
+        rope, rope_stride = new_rope.data_ptr(), new_rope.stride()[0]
     rows, rows_stride = (0, 0) if row_index is None else (row_index.data_ptr(), row_index.stride()[0])
     fp8, scales = (0, 0) if quantised is None else (_ptr(quantised[0]), _ptr(quantised[1]))
-    return _pack_decode(_ptr(q), q_seq_stride, q_head_stride, _view_bytes(view), table, max_blocks, _ptr(kv_len), _ptr(kv_begin),
+    return _pack_decode(q.data_ptr(), q_seq_stride, q_head_stride, bytes(view) if isinstance(view, PoolView) else _refuse_view(view), table, max_blocks, _ptr(kv_len), _ptr(kv_begin),
                       batch, heads, block_size, scale, _ptr(out), _ptr(lse), o, m, l, ws, ws_bytes, variant, max_ctas,
                       latent, latent_stride, rope, rope_stride, 1 if stable_tables else 0, rows, rows_stride, fp8, scales)
 
@@ -758,13 +758,13 @@ class Engine:
         cos_stride, sin_stride = cos.stride(), sin.stride()
         q_ptr, q_stride = (0, (0, 0)) if q_rope is None else (q_rope.data_ptr(), q_rope.stride())
         check(lib.b200kv_engine_layer_append(
-            self._h, layer, _ptr(kv_a), kv_a.stride()[0], _ptr(gamma), _ptr(cos),
-            cos_stride[0] if len(cos_stride) == 2 else 0, _ptr(sin), sin_stride[0] if len(sin_stride) == 2 else 0,
+            self._h, layer, kv_a.data_ptr(), kv_a.stride()[0], _ptr(gamma), cos.data_ptr(),
+            cos_stride[0] if len(cos_stride) == 2 else 0, sin.data_ptr(), sin_stride[0] if len(sin_stride) == 2 else 0,
             q_ptr, q_stride[0], q_stride[1], _stream_handle(stream)))
 
     def layer_attend(self, layer: int, q, out, out_fp8=None, out_scales=None, stream=None):
         q_stride = q.stride()
-        check(lib.b200kv_engine_layer_attend(self._h, layer, _ptr(q), q_stride[0], q_stride[1], _ptr(out), _ptr(out_fp8),
+        check(lib.b200kv_engine_layer_attend(self._h, layer, q.data_ptr(), q_stride[0], q_stride[1], _ptr(out), _ptr(out_fp8),
                                              _ptr(out_scales), _stream_handle(stream)))
 
     def end_step(self):
