@@ -127,8 +127,7 @@ struct TcParams {
 };
 
 // A bounded wait by all lanes of a warp together, behind an inline probe: a phase that is complete already (the usual case
-// for a tile's later slab groups) costs no call. 45.2 -> 44.2 us for 32 sequences of 4,096 tokens, 17.4 -> 16.9 us for one
-// of 8,192.
+// for a tile's later slab groups) costs no call: 0.8 % of a call over 32 sequences of 4,096 tokens, 1.2 % over one of 262,144.
 __device__ __forceinline__ bool WarpWait(uint32_t bar, uint32_t parity, Misc* misc, int32_t* status, int site) {
   if (__all_sync(0xffffffffu, ptx::MbarTestWait(bar, parity))) return true;
   return __all_sync(0xffffffffu, BoundedWait(bar, parity, misc, status, site));
@@ -1069,7 +1068,7 @@ __global__ void __launch_bounds__(kGroups == 1 ? 128 : 256, kResident)
   constexpr int kChunk = kGroupParts * kGroups;        // parts per chunk
   constexpr int kRounds = kGroupParts / 8;             // a warp works out the weights of 8 parts x 4 heads at a time
   constexpr int kSub = kPasses == 2 ? 4 : 8;           // parts whose data a thread has in flight
-  constexpr int kDvChunks = kLatent / kDv;             // 2 or 16
+  constexpr int kDvChunks = kLatent / kDv;             // 2, 4, 8 or 16
   constexpr int kQuads = kHeads / 4;
 
   const int tid = threadIdx.x;
@@ -1198,7 +1197,7 @@ __global__ void __launch_bounds__(kGroups == 1 ? 128 : 256, kResident)
     if (c0 != cf) __syncthreads();  // the previous chunk's weights and slots have been used
     if (tid < kChunk) s_slot[tid] = slot_of(c0 + tid);
     __syncthreads();
-      // This thread's parts of the chunk, kSub at a time.
+    // This thread's parts of the chunk, kSub at a time.
     float4 data[kSub][kPasses];
     auto load_sub = [&](int sub) {
 #pragma unroll

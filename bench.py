@@ -480,8 +480,8 @@ def measure_move_kernels(torch, b200kv, wl: Workload, hbm_peak: float, use_graph
         t = timeit(lambda i: b200kv.indexer_topk(q8, q_scale, w_idx, key8[i % 8], k_scale[i % 8], wl.table, wl.kv_len,
                                                  BLOCK, CONTEXT, 512, status=wl.status, variant=variant), 24)
         res[name] = {"sequences": BATCH, "tokens_per_sequence": CONTEXT, "index_heads": HEADS, "k": 512,
-                     "kernels": "score (FP8 tcgen05) + radix select" if variant == b200kv.INDEXER_TCGEN05
-                                else "score (fp32 chains on CUDA cores) + radix select",
+                     "kernels": "score (FP8 tcgen05) + selection" if variant == b200kv.INDEXER_TCGEN05
+                                else "score (fp32 chains on CUDA cores) + selection",
                      "us_per_launch": t * 1e6, "score_bytes": idx_bytes,
                      "gflop": 2.0 * BATCH * CONTEXT * HEADS * 128 * 1e-9,
                      "tflops": 2.0 * BATCH * CONTEXT * HEADS * 128 / t * 1e-12}

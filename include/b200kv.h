@@ -117,7 +117,7 @@ int32_t b200kv_gather(const b200kv_pool_view* pool, const int32_t* block_table, 
  */
 #define B200KV_DECODE_AUTO 0
 #define B200KV_DECODE_SIMT 1   /* CUDA-core kernel: any geometry                            */
-#define B200KV_DECODE_TCGEN05 2 /* tensor-core kernel: 64 heads, 512+64, block_size % 64 == 0 */
+#define B200KV_DECODE_TCGEN05 2 /* tensor-core kernels: 64 heads, 512+64, block_size % 64 == 0 (AUTO: any geometry) */
 
 typedef struct b200kv_decode_args {
   const void* q;
@@ -144,8 +144,9 @@ typedef struct b200kv_decode_args {
   /*
    * Append fused into the attention launch (tensor-core kernel, kv_begin null; both null = none): the new row
    * of sequence b, new_latent[b] (512 bf16) and new_rope[b] (64 bf16), row strides in elements (multiples of
-   * 8), is written to the pool at the sequence's last position kv_len[b] - 1, through the block table, by the
-   * CTA that attends over that position, before it reads the tile. The result equals b200kv_append with
+   * 8), is written to the pool at the sequence's last position kv_len[b] - 1, through the block table, by a
+   * CTA that attends over that position, and takes its place in the tile before that is attended over. The result equals
+   * b200kv_append with
    * slot_mapping[b] = block_table[b][(kv_len[b]-1) / block_size] * block_size + (kv_len[b]-1) % block_size
    * followed by the attention: the two stages the reference plans back to back
    * (src/pipeline/pipeline.cpp:226-249) as one launch. Sequences with kv_len 0 append nothing.
@@ -178,8 +179,8 @@ typedef struct b200kv_decode_args {
    * [batch][heads][16] E8M0, block-32 MX along a head's row, bit for bit what b200kv_mx_quant_e4m3 gives on `out`
    * viewed as [batch][heads * 512]: the reference's stage after attention (attn_quant,
    * src/pipeline/pipeline.cpp:250-258) as the epilogue of the kernel that writes `out`, instead of a launch of its
-   * own that reads `out` back. Needs `out` (not the partial_* form). The CUDA-core path runs the stand-alone
-   * quantiser behind the attention.
+   * own that reads `out` back. Needs `out` (not the partial_* form). The CUDA-core path (`B200KV_DECODE_SIMT`) runs the
+   * stand-alone quantiser behind the attention.
    */
   void* out_fp8;
   void* out_scale;
@@ -196,8 +197,8 @@ int32_t b200kv_mla_decode(const b200kv_decode_args* args, void* stream, b200kv_s
  * t = token_index[b][j], j < n_selected[b] (the rest -1; a token outside the table or the pool is recorded
  * as B200KV_DEV_BAD_BLOCK). b200kv_mla_decode then attends over exactly those rows when it is given
  * row_index = rows, row_index_stride = max_selected and kv_len = n_selected (tensor-core kernel for 64 heads), or,
- * equivalently, block_table = rows, max_blocks = max_selected and block_size = 1 (a table of single-row blocks,
- * which runs on the CUDA-core kernel). All arrays device int32.
+ * equivalently, block_table = rows, max_blocks = max_selected and block_size = 1 (a table of single-row blocks, of
+ * any number of heads). All arrays device int32.
  */
 int32_t b200kv_resolve_rows(const int32_t* block_table, int64_t max_blocks, int64_t block_size, const int32_t* token_index,
                             int64_t max_selected, const int32_t* n_selected, int64_t batch, int64_t pool_rows,

@@ -196,9 +196,10 @@ def test_simt_handles_other_head_counts():
     for heads in (8, 128):
         q = kvo.make_q(2, heads=heads)
         want, want_lse = kvo.mla_decode(q, pool, table, kv_len, bs, 1.0 / 24.0, use_double=True)
-        out, lse = run_decode(q, pool, table, kv_len, bs, 1.0 / 24.0, b200kv.DECODE_AUTO)
-        scenarios.check_attention(out, lse, kvo.bf16_to_f32(want).astype(np.float64), want_lse.astype(np.float64),
-                                  what=f"heads={heads}", strict_abs=True)
+        for variant in (b200kv.DECODE_SIMT, b200kv.DECODE_AUTO):
+            out, lse = run_decode(q, pool, table, kv_len, bs, 1.0 / 24.0, variant)
+            scenarios.check_attention(out, lse, kvo.bf16_to_f32(want).astype(np.float64), want_lse.astype(np.float64),
+                                      what=f"heads={heads}", strict_abs=True)
 
 
 def test_decode_reports_bad_block_without_faulting():
@@ -326,9 +327,9 @@ def test_gathered_rows_outside_the_pool_are_recorded_not_read():
 def test_output_quantised_by_the_launch_that_writes_it(case):
     """out_fp8 / out_scale: the MX quantisation of the attention output as the epilogue of the merge kernel (and,
     for sequences a single CTA covers, of the read-back of what the decode kernel wrote). Bit for bit the
-    stand-alone quantiser on `out`, which is bit for bit the oracle's. Sequences cut over several CTAs (the
-    32-CTAs-per-sequence merge), a few long ones (the 256-CTAs-per-sequence merge), many short ones with empty
-    ones among them (whole sequences per CTA), and the CUDA-core path (quantiser behind the attention)."""
+    stand-alone quantiser on `out`, which is bit for bit the oracle's. Sequences cut over several CTAs, a few long ones
+    (another shape of the merge), many short ones with empty ones among them, and the CUDA-core path (quantiser behind the
+    attention)."""
     from gpu_util import from_dev_bf16, status_ok, to_dev_bf16, to_dev_i32
 
     bs = 64

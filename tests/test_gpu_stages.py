@@ -240,9 +240,8 @@ def _indexer_inputs(B, H, lens, bs, seed):
 @pytest.mark.parametrize("lens,k", [([4096, 300, 5000, 17, 0, 9000], 512), ([70, 64], 2048), ([12000], 100),
                                     ([9000, 8193, 8192, 40000], 2048)])
 def test_indexer_selection_matches_oracle_bit_for_bit(lens, k):
-    """Exact scores: the selection equals the oracle's, position for position. Sequences of up to 8,192 tokens are
-    selected by one CTA, longer ones in two levels (the best of every 8,192-token chunk, then the best of those):
-    lengths on both sides of the chunk edge, a chunk that holds fewer tokens than k, five chunks."""
+    """Exact scores: the selection equals the oracle's, position for position. Several cluster sizes (a CTA for every 4,096
+    tokens of the longest sequence), short sequences beside long ones, fewer tokens than k, an empty sequence."""
     B, H, bs = len(lens), 64, 64
     q, qs, w, key, ks, table, kv_len = _indexer_inputs(B, H, lens, bs, seed=11 + k)
     # ties on purpose: two tokens with identical keys and scales
@@ -470,7 +469,7 @@ def test_sparse_attention_pipeline_indexer_then_resolved_rows_then_decode():
                       workspace=ws, variant=b200kv.DECODE_TCGEN05, status=status, row_index=rows)
     status_ok(status)
     scenarios.check_attention(from_dev_bf16(out), lse.cpu().numpy(), ref_out, ref_lse, what="sparse pipeline, gathered")
-    # and as a table of single-row blocks on the CUDA-core kernel
+    # and as a table of single-row blocks
     out, lse = run_decode(q, pool, exp_rows, exp_n, 1, 1.0 / 24.0, b200kv.DECODE_AUTO)
     scenarios.check_attention(out, lse, ref_out, ref_lse, what="sparse pipeline")
 
