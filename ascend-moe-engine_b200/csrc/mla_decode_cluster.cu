@@ -21,9 +21,9 @@
 // spin instead of parking 1 %.)
 //
 // Measured (B200, graph of layers, us a layer): one sequence of 129 tokens with the append 16.4 (flat kernel and merge)
-// -> 7.9, of which 0.9 from the previous layer's end to the wait's return, 0.4 issue, 1.1 latency, 1.1 QK behind the
+// -> 7.7, of which 0.9 from the previous layer's end to the wait's return, 0.4 issue, 1.1 latency, 1.1 QK behind the
 // 91 KB that a CTA takes in, 0.6 softmax, 0.7 PV, 0.6 + 0.9 exchange, 1.0 merge; 16 sequences of 300 .. 4,096 tokens in
-// pages of 16 rows 360 (CUDA-core kernel) -> 53.6; 32 sequences of up to 2,048 tokens with 16 heads 373 -> 25.4.
+// pages of 16 rows 361 (CUDA-core kernel) -> 51.3; 32 sequences of up to 2,048 tokens with 16 heads 373 -> 26.1.
 //
 // Roles as in the flat kernel: warps 0-3 softmax, 4 producer, 5 QK, 6 PV; all eight warps take part in the exchange and
 // the merge. Every wait is bounded; a CTA
