@@ -351,3 +351,17 @@ def test_two_sequences_of_up_to_4096_tokens():
         out, lse = _decode_dev(q, pool, table, lens, 64)
         assert ((out.double() - want).abs() <= 2e-3 + 1e-2 * want.abs().amax(dim=2, keepdim=True)).all()
         assert (lse.double() - want_lse).abs().max() <= 1e-4
+
+
+@pytest.mark.parametrize("batch,tiles", [(1, 32), (2, 64), (5, 32), (12, 16), (30, 16), (60, 12), (140, 8)])
+def test_which_kernel_takes_a_call(batch, tiles):
+    """Up to so many tiles in the longest sequence a table can hold, a call runs in clusters, which leave the workspace alone;
+    with one more it runs in the kernel for many tiles, whose sequences are cut and leave partials there."""
+    for more in (0, 1):
+        q, pool, table, lens, rows = _case([64 * (tiles + more)] * batch, 64)
+        ws = torch.full((b200kv.decode_workspace_bytes(batch),), 0x5A, dtype=torch.uint8, device="cuda")
+        status = b200kv.new_status()
+        out = torch.empty((batch, 64, 512), dtype=torch.bfloat16, device="cuda")
+        b200kv.mla_decode(q, b200kv.pool_view(pool), table, lens, 64, 1.0 / 24.0, out=out, workspace=ws, status=status)
+        status_ok(status)
+        assert bool((ws == 0x5A).all()) == (more == 0)
