@@ -21,7 +21,7 @@
 // spin instead of parking 1 %.)
 //
 // Measured (B200, graph of layers, us a layer): one sequence of 129 tokens with the append 16.4 (flat kernel and merge)
-// -> 7.7, of which 0.9 from the previous layer's end to the wait's return, 0.4 issue, 1.1 latency, 1.1 QK behind the
+// -> 7.6, of which 0.9 from the previous layer's end to the wait's return, 0.4 issue, 1.1 latency, 1.1 QK behind the
 // 91 KB that a CTA takes in, 0.6 softmax, 0.7 PV, 0.6 + 0.9 exchange, 1.0 merge; 16 sequences of 300 .. 4,096 tokens in
 // pages of 16 rows 361 (CUDA-core kernel) -> 51.3; 32 sequences of up to 2,048 tokens with 16 heads 373 -> 26.1.
 //
@@ -580,14 +580,21 @@ __global__ void __launch_bounds__(kThreads, 1)
     const int head0 = warp * 16 + quad_row;  // and head0 + 8: this thread's two rows
     const uint32_t lane_base = static_cast<uint32_t>(warp * 32) << 16;
     const bool has_rows = warp * 16 < share.heads;  // otherwise the warp only keeps step with the others
-    // The four warps leave the loop on the same tile: a wait can run out for one of them and not for another, and whoever
-    // stayed would stand at the named barriers for good. So a warp whose wait ran out goes on, with whatever the
-    // accumulators hold (the result is void), asks for the rescaling path, and there all four leave on one vote. The usual
-    // path carries no vote of its own.
+    // The four warps leave the loop together: a wait can run out for one of them and not for another, and whoever stayed
+    // would stand at the named barriers for good. So a warp whose wait ran out goes through the barriers that the others
+    // will come to: it asks for the rescaling path, where all four leave on one vote. The usual path carries no vote.
+    auto leave_with_the_others = [&](bool at_the_vote) {
+      if (!at_the_vote) ptx::NamedBarrierOr(1, kSoftmaxThreads, true);
+      ptx::NamedBarrierOr(2, kSoftmaxThreads, true);
+    };
     for (int i = 0; i < n; ++i) {
       const int buf = kSplitP ? 0 : i & 1, stage = i % kStages;
       const int valid = min(kTile, len - (share.t_lo + i) * kTile);
-      if (ok) ok = WarpWait(bar(&misc->s_full[buf]), (kSplitP ? i : i >> 1) & 1, misc, p.status, 230);
+      ok = WarpWait(bar(&misc->s_full[buf]), (kSplitP ? i : i >> 1) & 1, misc, p.status, 230);
+      if (!ok) {
+        leave_with_the_others(false);
+        break;
+      }
       ptx::TcFenceAfterSync();
       uint32_t sr[32];
       if (has_rows) {
@@ -668,15 +675,19 @@ __global__ void __launch_bounds__(kThreads, 1)
         sum += __shfl_xor_sync(0xffffffffu, sum, 2);
         l_run[r] += sum;
       }
-      const bool any_rescale = ptx::NamedBarrierOr(1, kSoftmaxThreads, rescale || !ok);
-      if (ok && i > 0 && (any_rescale || kSplitP)) {
+      const bool any_rescale = ptx::NamedBarrierOr(1, kSoftmaxThreads, rescale);
+      if (i > 0 && (any_rescale || kSplitP)) {
         // PV of the previous tile must have drained: before its accumulators are rescaled (rare), and before the one
         // buffer of P's low term is written again. (It ran under this tile's exponentials.)
         ok = WarpWait(bar(&misc->kv_empty[(i - 1) % kStages][kGroups - 1]), ((i - 1) / kStages) & 1, misc, p.status, 231);
+        if (!ok) {
+          if (any_rescale || i + 1 < n) leave_with_the_others(any_rescale);  // (after the last tile nobody comes to them)
+          break;
+        }
         ptx::TcFenceAfterSync();
       }
       if (any_rescale) {
-        if (ptx::NamedBarrierOr(2, kSoftmaxThreads, !ok)) {
+        if (ptx::NamedBarrierOr(2, kSoftmaxThreads, false)) {
           ok = false;
           break;
         }

@@ -1,7 +1,8 @@
 """Warps that share named barriers leave their loops together. The bounded waits of the tensor-core kernels can run out for
 one warp and not for another; named barriers have no bound, so a warp that left on its own verdict would leave the others
 standing at the next one for good. Such a run-out cannot be produced on demand, so the rule is checked where it is written:
-between a wait's verdict and the barrier that votes on it, nothing leaves the loop."""
+between a wait's verdict and the barrier that votes on it, or the barriers that the warps which stay will come to, nothing
+leaves the loop."""
 import os
 import re
 
@@ -17,7 +18,8 @@ ROLES = {
 }
 
 EVENT = re.compile(
-    r"(?P<vote>NamedBarrierOr\([^;{]*!ok\))"        # a barrier over the role's warps that carries their verdicts
+    # a barrier over the role's warps that carries their verdicts, or a warp going through those that the others come to
+    r"(?P<vote>NamedBarrierOr\([^;{]*!ok\)|leave_with_the_others\()"
     r"|(?P<wait>\bok = [^;]*Wait\()"               # a bounded wait's verdict
     r"|(?P<leave>\bbreak;|\breturn;|\bfor \([^;{]*;[^;{]*\bok\b[^;{]*;)")
 
@@ -49,3 +51,4 @@ def test_warps_that_share_a_barrier_leave_together(name):
 def test_the_rule_catches_an_exit_on_a_warps_own_verdict():
     assert undecided_exits("ok = WarpWait(a); if (!ok) break; NamedBarrierOr(1, 128, r);") == ["break;"]
     assert undecided_exits("ok = WarpWait(a); v = NamedBarrierOr(1, 128, r || !ok); if (v) break;") == []
+    assert undecided_exits("ok = WarpWait(a); if (!ok) { leave_with_the_others(false); break; }") == []
