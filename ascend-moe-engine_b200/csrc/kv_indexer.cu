@@ -157,10 +157,8 @@ constexpr int kFewTokens = 128;  // up to so many keys are ordered by comparing 
 // 20,000 pairs a us. (512 keys in groups of 64 / 128 / 256 equal scores, one CTA: 1.6 / 3.2 / 6.0 us compared.)
 constexpr uint32_t kComparisonsPerKey = 100;
 // What SortKeys makes of a list of so many keys: a power of two, four keys to each thread of a warp at least.
-__host__ __device__ constexpr uint32_t PaddedKeys(uint32_t keys) {
-  uint32_t padded = 128;
-  while (padded < keys) padded <<= 1;
-  return padded;
+__device__ __forceinline__ uint32_t PaddedKeys(uint32_t keys) {
+  return keys <= 128 ? 128u : 1u << (32 - __clz(static_cast<int>(keys - 1)));
 }
 
 struct SelectParams {
